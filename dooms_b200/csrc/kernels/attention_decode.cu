@@ -35,37 +35,31 @@ using namespace dooms::cuda::attn_decode;
 
 namespace {
 
-template <int D, int GP>
+template <int D, int GP, int STAGES>
 __global__ void __launch_bounds__(kThreads) k_attention_decode(const AttnDecodeParams pp) {
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_trigger();
-    if (pp.l2_hint) {
-        // The cached keys and values of earlier positions do not depend on the projection that runs before this kernel. While that projection's last
-        // blocks drain, ask for this block's range of both caches to be brought to L2 (a hint: nothing is read into the SM). The position is read before
-        // the kernel that may still be writing it is known to be complete, so it can be one step old; that shifts the hinted range by one row at most.
-        const int pos = __ldcg(&pp.st->pos);
-        const int n_keys = pp.n_keys_fixed > 0 ? pp.n_keys_fixed : pos + 1;
-        const int tiles_total = (n_keys + kTileKeys - 1) / kTileKeys, tiles_per = (tiles_total + pp.splits - 1) / pp.splits;
-        const int j_begin = min(n_keys, int(blockIdx.y) * tiles_per * kTileKeys), j_end = min(n_keys, j_begin + tiles_per * kTileKeys);
-        constexpr int LINES = D * 2 / 128 > 0 ? D * 2 / 128 : 1;      // 128-byte lines per cached row of one head
-        if (pos >= 0 && pos < (1 << 28)) {
-            for (int i = threadIdx.x; i < (j_end - j_begin) * LINES; i += kThreads) {
-                const int64_t at = int64_t(j_begin + i / LINES) * pp.s.kv_stride + int(blockIdx.x) * D + (i % LINES) * 64;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(pp.kc + at));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(pp.vc + at));
-            }
-        }
-    }
-    pdl_wait();
-    attention_decode_body<D, GP, true>(pp, int(blockIdx.x), int(blockIdx.y), int(gridDim.y), int(blockIdx.z), smem);
+    if (!pp.cache_ready) pdl_wait();
+    attention_decode_body<D, GP, true, STAGES>(pp, int(blockIdx.x), int(blockIdx.y), int(blockIdx.z), smem);
+}
+
+// Heads of 128 on a context of which a range holds one pair of tiles at most: two stages are all such a block uses, and 74 KB instead of 143 leave it room beside
+// the projection in front, so that its fetches are early (the 8B shape at 60 keys: 10.3 us to 6.0). Longer ranges want the second pair on its way (the 32B shape
+// at 8200 keys, ranges of four pairs: 24.1 us with four stages, 28.4 with two, also with twice as many blocks).
+template <int D, int GP, int STAGES>
+cudaError_t launch_staged(const AttnDecodeParams & p, cudaStream_t stream) {
+    constexpr size_t smem = attention_decode_smem_bytes<D, GP, STAGES>();
+    static std::atomic<uint64_t> configured{0};
+    if (const cudaError_t e = allow_dynamic_smem(k_attention_decode<D, GP, STAGES>, int(smem), configured); e != cudaSuccess) return e;
+    return launch_pdl(k_attention_decode<D, GP, STAGES>, dim3(p.s.n_head_kv, p.splits, p.b_slot ? unsigned(p.b_rows) : 1u), dim3(kThreads), smem, stream, p);
 }
 
 template <int D, int GP>
 cudaError_t launch_one(const AttnDecodeParams & p, cudaStream_t stream) {
-    constexpr size_t smem = attention_decode_smem_bytes<D, GP>();
-    static std::atomic<uint64_t> configured{0};
-    if (const cudaError_t e = allow_dynamic_smem(k_attention_decode<D, GP>, int(smem), configured); e != cudaSuccess) return e;
-    return launch_pdl(k_attention_decode<D, GP>, dim3(p.s.n_head_kv, p.splits, p.b_slot ? unsigned(p.b_rows) : 1u), dim3(kThreads), smem, stream, p);
+    if constexpr (D > 64) {
+        if (p.cache_ready && p.cache_ready <= p.splits * 2 * kTileKeys) return launch_staged<D, GP, 2>(p, stream);
+    }
+    return launch_staged<D, GP, kStagesFull>(p, stream);
 }
 
 template <int D>
@@ -92,12 +86,11 @@ int attention_gqa_splits(int n_head_kv, int n_ctx) {
 }
 
 cudaError_t launch_attention_gqa(const float * qkv, void * kc, void * vc, float * part, const DevState * st, const double * inv_freq, int n_keys_fixed,
-                                 int splits, const AttnShape & s, int * counters, float * out, void * xq, cudaStream_t stream, const void * rope_cs) {
-    if (!attention_gqa_supported(s) || (!inv_freq && n_keys_fixed < 1) || (counters && !out) || (xq && !counters)) return cudaErrorInvalidValue;
+                                 int splits, const AttnShape & s, int * counters, float * out, void * xq, cudaStream_t stream, const void * rope_cs, int cache_keys) {
+    if (!attention_gqa_supported(s) || (!inv_freq && n_keys_fixed < 1) || (counters && !out) || (xq && !counters) || cache_keys < 0 || (cache_keys && (!st || !inv_freq))) return cudaErrorInvalidValue;
     AttnDecodeParams p{qkv, static_cast<__half *>(kc), static_cast<__half *>(vc), part, st, inv_freq, n_keys_fixed, splits, s, counters, out,
                        static_cast<uint8_t *>(xq), static_cast<const float2 *>(rope_cs), nullptr, nullptr, 0, 0, 0, nullptr, 0};
-    static const bool hint = [] { const char * e = getenv("DOOMS_ATTN_L2_HINT"); return !(e && *e == '0'); }();
-    p.l2_hint = (hint && st && inv_freq) ? 1 : 0;
+    p.cache_ready = cache_keys;
     return s.head_dim == 64 ? launch_group<64>(p, s.n_head / s.n_head_kv, stream) : launch_group<128>(p, s.n_head / s.n_head_kv, stream);
 }
 

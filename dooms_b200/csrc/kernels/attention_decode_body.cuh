@@ -5,6 +5,7 @@
 #include <math_constants.h>
 
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "xsplit.cuh"
 
@@ -16,7 +17,7 @@ using namespace dooms::dev;
 
 constexpr int kThreads = 256;
 constexpr int kTileKeys = 64;
-constexpr int kStages = 4;      // two pairs of tiles: the block's 8 warps work on one pair while the next is on its way
+constexpr int kStagesFull = 4;      // two pairs of tiles: the block's 8 warps work on one pair while the next is on its way
 
 struct AttnDecodeParams {
     const float * qkv;        // the new token's row: query heads, then key heads, then value heads
@@ -41,7 +42,10 @@ struct AttnDecodeParams {
     int64_t slot_elems;       // f16 elements between the caches of consecutive slots
     int64_t part_row_floats;  // floats of `part` per row
     __half * out16;           // optional: the merged rows as f16 as well ([row][n_head * head_dim]), the tensor-core GEMM's operand
-    int l2_hint;              // single-row decode: before waiting for the projection in front of it, a block asks for its range of the caches to be brought to L2
+    // Single-row decode inside a step whose position was final before this kernel could start (launch_attention_gqa): the cached keys and values of earlier
+    // positions do not depend on the projection in front of this kernel, so a block asks for its range before it waits for that projection. The row of the
+    // new position is whatever the cache held; it is overwritten in shared memory once the projection is done, as it always was.
+    int cache_ready;          // the positions the caches have room for (0: not so)
 };
 
 __device__ __forceinline__ void cp16(uint32_t dst, const void * src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
@@ -69,10 +73,10 @@ __device__ __forceinline__ void split_h2(float x, float y, uint32_t & hi, uint32
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
-// The work of one block of kThreads threads: key/value head `kvh`, range `split` of `n_splits`, row `row` of a batched step (0 otherwise), with `smem`
+// The work of one block of kThreads threads: key/value head `kvh`, range `split`, row `row` of a batched step (0 otherwise), with `smem`
 // (attention_decode_smem_bytes<D, GP>(), 128-byte aligned) as its staging memory. WHOLE = true: the calling block has exactly kThreads threads and its
 // barriers are __syncthreads(); false: the first kThreads threads of a larger block run this while the others do not, so the barriers are the named
-// barrier 1 over kThreads threads. Inputs written earlier in the same launch (the fused decode step calls this right after a grid-wide barrier) are read
+// barrier 1 over kThreads threads. With cache_ready the body itself waits for the kernel in front (pdl_wait), after its first fetches. Inputs written earlier in the same launch (the fused decode step calls this right after a grid-wide barrier) are read
 // with loads that bypass L1.
 // D: head_dim (64 or 128). GP: query heads per key/value head, rounded up to 1, 2, 4 or 8.
 template <bool WHOLE>
@@ -85,11 +89,11 @@ __device__ __forceinline__ void attn_bar() {
 // numbers (value and rounding error, two MMAs), so the products are as exact as the f32 arithmetic they replace: one position per call keeps the
 // reference's token-by-token tolerance (tests/unit/test_metal_llama_decoder.cpp:335). The 8 warps take 16 keys each of a pair of 64-key tiles with their
 // own running maximum / sum / output and are merged through shared memory at the end of the range.
-template <int D, int GP>
-constexpr size_t attention_decode_smem_bytes() { return size_t(16) * (D + 8) * 2 + size_t(kStages) * kTileKeys * 2 * (D * 2 + 16); }
+template <int D, int GP, int STAGES = kStagesFull>
+constexpr size_t attention_decode_smem_bytes() { return size_t(16) * (D + 8) * 2 + size_t(STAGES) * kTileKeys * 2 * (D * 2 + 16); }
 
-template <int D, int GP, bool WHOLE>
-__device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & pp, const int kvh, const int split, const int n_splits, const int row, uint8_t * smem) {
+template <int D, int GP, bool WHOLE, int kStages = kStagesFull>
+__device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & pp, const int kvh, const int split, const int row, uint8_t * smem) {
     constexpr int LD = D + 8;                           // halves between staged rows: 16 bytes of padding keep the 8 rows of an ldmatrix on different banks
     constexpr int KP = LD * 2, VP = LD * 2;             // the same in bytes
     constexpr int STAGE = kTileKeys * (KP + VP);
@@ -121,9 +125,13 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
     const bool fuse = p.inv_freq != nullptr;
     const int pos = !fuse ? 0 : pp.b_slot ? row_pos : p.st->pos;
     const int n_keys = p.n_keys_fixed > 0 ? p.n_keys_fixed : pos + 1;
-    // ranges of whole tiles, the same for every head: at least one tile per range, so short contexts leave the later ranges empty
+    // Ranges of whole tiles, the same for every head. A range of two tiles takes as long as one of one tile (four warps each), so ranges are whole pairs, and only the first `used` of the p.splits ranges hold keys. The blocks of
+    // the others leave at once and the merge reads `used` results (with one range there is nothing to merge): on the 0.5B shape, 2 key/value heads and so
+    // 74 ranges, a context of 39 keys would otherwise gather 73 empty results and one of 512 keys 66.
     const int tiles_total = (n_keys + kTileKeys - 1) / kTileKeys;
-    const int tiles_per = (tiles_total + p.splits - 1) / p.splits;
+    const int tiles_per = ((tiles_total + p.splits - 1) / p.splits + 1) & ~1;
+    const int used = (tiles_total + tiles_per - 1) / tiles_per;
+    if (split >= used && p.counters) return;      // (without counters the caller's combine reads every range)
     const int j_begin = min(n_keys, split * tiles_per * kTileKeys), j_end = min(n_keys, j_begin + tiles_per * kTileKeys);
     const int ntiles = (j_end - j_begin + kTileKeys - 1) / kTileKeys;
 
@@ -146,6 +154,16 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
     for (int i = 0; i < kStages; i++) {
         if (i < ntiles) fetch(i);
         cp_commit();
+    }
+    if (pp.cache_ready) {
+        // what does not fit the stages is asked for into L2
+        constexpr int LINES = D * 2 / 128 > 0 ? D * 2 / 128 : 1;      // 128-byte lines per cached row of one head
+        for (int i = tid; i < (j_end - j_begin - kStages * kTileKeys) * LINES; i += kThreads) {
+            const int64_t at = int64_t(j_begin + kStages * kTileKeys + i / LINES) * p.s.kv_stride + kvh * D + (i % LINES) * 64;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.kc + at));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.vc + at));
+        }
+        pdl_wait();
     }
 
     // the group's queries, rotated (when asked), each as an f16 value and the f16 rounding error of that value
@@ -292,9 +310,35 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
     #pragma unroll
     for (int n = 0; n < D / 8; n++) *reinterpret_cast<float2 *>(res + (warp * 8 + g) * RS + 2 + n * 8 + 2 * t) = make_float2(o[n][0], o[n][1]);
     attn_bar<WHOLE>();
+    auto weight = [&](int w, int hq, float M) { const float mw = res[(w * 8 + hq) * RS]; return mw == -CUDART_INF_F ? 0.f : expf(mw - M); };
+    auto finish = [&](int hq, int d, float r) {      // a warp holds 32 consecutive elements of one head
+        p.out[(kvh * G + hq) * D + d] = r;
+        if (p.out16) p.out16[(kvh * G + hq) * D + d] = __float2half_rn(r);
+        if (p.xq) split_block(r, lane, ((kvh * G + hq) * D + d) / 32, p.s.n_head * D / 32, p.xq);
+    };
+    if (used == 1 && p.counters) {
+        // one range: its result is the head's, no other block is involved
+        #pragma unroll
+        for (int it = 0; it < MERGE_IT; it++) {
+            const int idx = tid + it * kThreads;
+            const int hq = idx / D, d = idx % D;
+            if (idx < GP * D && hq < G) {
+                float M = -CUDART_INF_F, l = 0.f, v = 0.f;
+                #pragma unroll
+                for (int w = 0; w < 8; w++) M = fmaxf(M, res[(w * 8 + hq) * RS]);
+                #pragma unroll
+                for (int w = 0; w < 8; w++) {
+                    const float f = weight(w, hq, M);
+                    l += res[(w * 8 + hq) * RS + 1] * f;
+                    v += res[(w * 8 + hq) * RS + 2 + d] * f;
+                }
+                finish(hq, d, v / l);
+            }
+        }
+        return;
+    }
     float m_run = -CUDART_INF_F, l_run = 0.f;
     float acc[OUT_IT][2];
-    auto weight = [&](int w, int hq, float M) { const float mw = res[(w * 8 + hq) * RS]; return mw == -CUDART_INF_F ? 0.f : expf(mw - M); };
     if (warp < GP) {
         #pragma unroll
         for (int w = 0; w < 8; w++) m_run = fmaxf(m_run, res[(w * 8 + warp) * RS]);
@@ -320,7 +364,7 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
         }
     }
     cp_wait<0>();
-    // partial results (an empty range leaves sum = 0, which the merge skips)
+    // partial results
     #pragma unroll
     for (int it = 0; it < OUT_IT; it++) {
         const int idx = tid + it * kThreads;
@@ -345,15 +389,15 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
     attn_bar<WHOLE>();
     if (tid == 0) {
         const int done = atomicAdd(p.counters + kvh, 1);
-        is_last = done == n_splits - 1;
+        is_last = done == used - 1;
         if (is_last) p.counters[kvh] = 0;          // ready for the next step; nobody else touches it any more in this launch
     }
     attn_bar<WHOLE>();
     if (!is_last) return;
     __threadfence();
     // weights of the ranges, per head: warp w takes head w (the stage buffers are free now and hold them)
-    float * wts = reinterpret_cast<float *>(stages);            // [GP][splits]
-    float * tot = wts + GP * p.splits;                          // [GP]
+    float * wts = reinterpret_cast<float *>(stages);            // [GP][used]
+    float * tot = wts + GP * used;                              // [GP]
     // Every load of the merge is issued before anything waits on one: the partial results sit in L2, a round trip there costs more than all the
     // arithmetic of the merge, and loops that load and add split by split would pay it once per split.
     if (warp < G) {
@@ -363,7 +407,7 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
         #pragma unroll
         for (int k = 0; k < kPerLane; k++) {
             const int sp = lane + 32 * k;
-            ml[k] = sp < p.splits ? __ldcg(reinterpret_cast<const float2 *>(base + sp * (2 + D))) : make_float2(-CUDART_INF_F, 0.f);
+            ml[k] = sp < used ? __ldcg(reinterpret_cast<const float2 *>(base + sp * (2 + D))) : make_float2(-CUDART_INF_F, 0.f);
         }
         float mx = -CUDART_INF_F;
         #pragma unroll
@@ -374,9 +418,9 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
         #pragma unroll
         for (int k = 0; k < kPerLane; k++) {
             const int sp = lane + 32 * k;
-            if (sp < p.splits) {
+            if (sp < used) {
                 const float w = ml[k].y > 0.f ? expf(ml[k].x - mx) : 0.f;      // an empty range weighs nothing
-                wts[warp * p.splits + sp] = w;
+                wts[warp * used + sp] = w;
                 total += ml[k].y * w;
             }
         }
@@ -389,7 +433,7 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
     float merged[MERGE_IT];
     #pragma unroll
     for (int it = 0; it < MERGE_IT; it++) merged[it] = 0.f;
-    for (int sp0 = 0; sp0 < p.splits; sp0 += kChunk) {
+    for (int sp0 = 0; sp0 < used; sp0 += kChunk) {
         #pragma unroll
         for (int it = 0; it < MERGE_IT; it++) {
             const int idx = tid + it * kThreads;            // (head, element): a warp holds 32 consecutive elements of one head
@@ -397,7 +441,7 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
             const bool mine = idx < GP * D && hq < G;
             const float * col = p.part + int64_t(kvh * G + (mine ? hq : 0)) * p.splits * (2 + D) + 2 + d;
             #pragma unroll
-            for (int k = 0; k < kChunk; k++) v[it][k] = (mine && sp0 + k < p.splits) ? __ldcg(col + (sp0 + k) * (2 + D)) : 0.f;
+            for (int k = 0; k < kChunk; k++) v[it][k] = (mine && sp0 + k < used) ? __ldcg(col + (sp0 + k) * (2 + D)) : 0.f;
         }
         if (sp0 == 0) attn_bar<WHOLE>();                                // the weights are in shared memory (the first chunk's loads are already on their way)
         #pragma unroll
@@ -405,9 +449,9 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
             const int idx = tid + it * kThreads;
             const int hq = idx / D;
             if (idx < GP * D && hq < G) {
-                const float * w = wts + hq * p.splits + sp0;
+                const float * w = wts + hq * used + sp0;
                 #pragma unroll
-                for (int k = 0; k < kChunk; k++) if (sp0 + k < p.splits) merged[it] += v[it][k] * w[k];      // an empty range's values are finite (zeros), its weight 0
+                for (int k = 0; k < kChunk; k++) if (sp0 + k < used) merged[it] += v[it][k] * w[k];      // an empty range's values are finite (zeros), its weight 0
             }
         }
     }
@@ -415,12 +459,7 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
     for (int it = 0; it < MERGE_IT; it++) {
         const int idx = tid + it * kThreads;
         const int hq = idx / D, d = idx % D;
-        if (idx < GP * D && hq < G) {
-            const float r = merged[it] / tot[hq];
-            p.out[(kvh * G + hq) * D + d] = r;
-            if (p.out16) p.out16[(kvh * G + hq) * D + d] = __float2half_rn(r);
-            if (p.xq) split_block(r, lane, ((kvh * G + hq) * D + d) / 32, p.s.n_head * D / 32, p.xq);
-        }
+        if (idx < GP * D && hq < G) finish(hq, d, merged[it] / tot[hq]);
     }
 }
 

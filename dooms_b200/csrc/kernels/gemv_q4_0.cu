@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_decode_layers(const FusedA
             grid_barrier(gb);                              // q, k and v of this layer are complete
             const int nkv = cur.a.s.n_head_kv;
             if (threadIdx.x < attn_decode::kThreads && block < nkv * cur.a.splits) {
-                attn_decode::attention_decode_body<D, GP, false>(cur.a, block % nkv, block / nkv, cur.a.splits, 0, smem);
+                attn_decode::attention_decode_body<D, GP, false>(cur.a, block % nkv, block / nkv, 0, smem);
             }
         }
         __syncthreads();                                   // the phase's shared memory is free, the next phase's description is in place

@@ -249,7 +249,11 @@ __global__ void k_add(float * x, const float * y, int64_t n) {
 
 // cs[i] = (cos, sin)(st->pos * inv_freq[i]) for the head_dim / 2 rotary pairs, in double precision, rounded to f32: what every head of every layer of one
 // decode step rotates by, computed once per step instead of in every attention launch.
+// It waits for everything before it first and only then lets the kernels after it start: whatever they read before their own wait (the position, cache rows
+// of earlier steps) is final by then.
 __global__ void k_rope_table(const DevState * st, const double * inv_freq, float2 * cs, int pairs, unsigned * zero) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0 && zero) { zero[0] = 0u; zero[32] = 0u; }      // the fused step's barrier words
     if (i >= pairs) return;
@@ -587,8 +591,7 @@ cudaError_t launch_add(float * x, const float * y, int64_t n, cudaStream_t strea
 
 cudaError_t launch_rope_table(const DevState * st, const double * inv_freq, void * cs, int head_dim, cudaStream_t stream, unsigned * zero) {
     const int pairs = head_dim / 2;
-    k_rope_table<<<(pairs + 127) / 128, 128, 0, stream>>>(st, inv_freq, static_cast<float2 *>(cs), pairs, zero);
-    return cudaGetLastError();
+    return launch_pdl(k_rope_table, dim3((pairs + 127) / 128), dim3(128), 0, stream, st, inv_freq, static_cast<float2 *>(cs), pairs, zero);
 }
 
 cudaError_t launch_rope_store(float * qkv, void * kc, void * vc, const DevState * st, const double * inv_freq, int M, const AttnShape & s, cudaStream_t stream) {

@@ -87,7 +87,11 @@ int attention_gqa_splits(int n_head_kv, int n_ctx);
 // With counters (n_head_kv zeroed ints, left zeroed) the last block of each key/value head merges the ranges itself into out (and xq): no combine launch.
 cudaError_t launch_attention_gqa(const float * qkv, void * kc, void * vc, float * part, const DevState * st, const double * inv_freq, int n_keys_fixed,
                                  int splits, const AttnShape & s, int * counters, float * out, void * xq, cudaStream_t stream,
-                                 const void * rope_cs = nullptr);   // rope_cs: launch_rope_table's output for st->pos, used instead of computing the angles
+                                 const void * rope_cs = nullptr,    // launch_rope_table's output for st->pos, used instead of computing the angles
+                                 // the caller vouches that st->pos and the cache rows before it were final before this kernel could start: a launch_rope_table
+                                 // earlier in the stream orders them (its dependents start only after its own wait); rows may then be read before the wait. The value: the
+                                 // positions the caches have room for.
+                                 int cache_keys = 0);
 
 // ---- one decode step over several sequences at once ----
 // Row r of the step belongs to the KV-cache slot slot[r] (negative: the row is idle, every kernel skips it) and sits at position pos[r] of that
