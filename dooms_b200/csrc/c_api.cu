@@ -669,6 +669,13 @@ DOOMS_CUDA_API int32_t dooms_cuda_matvec(int32_t dtype, const void * d_w, const 
     }
     if (rows == 0) return DOOMS_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if ((reinterpret_cast<uintptr_t>(d_x) & 15u) == 0 && cuda::gemv_short_supported(dtype, d_w, rows, cols, 1)) {
+        const cuda::ShortMatrix m{dtype, d_w, nullptr, rows, d_y, d_bias};
+        return launch_result(cuda::launch_gemv_short(&m, 1, nullptr, d_x, nullptr, 0.f, cols, flags, st), "matvec");
+    }
+    if ((reinterpret_cast<uintptr_t>(d_x) & 15u) == 0 && cuda::gemv_tall_supported(dtype, d_w, rows, cols)) {
+        return launch_result(cuda::launch_gemv_tall(dtype, d_w, nullptr, d_x, nullptr, 0.f, d_y, d_bias, rows, cols, flags, st), "matvec");
+    }
     if (dtype == DOOMS_Q4_0 && cuda::gemv_q4_0_supported(d_w, rows, cols)) return fast_q4_0(d_w, nullptr, d_x, d_y, d_bias, rows, cols, flags, false, st, "matvec");
     if (dtype == DOOMS_Q4_K && cuda::gemv_q4_k_supported(d_w, rows, cols)) return fast_q4_0(d_w, nullptr, d_x, d_y, d_bias, rows, cols, flags, true, st, "matvec");
     if (dtype == DOOMS_Q6_K && cuda::gemv_q6_k_supported(d_w, rows, cols)) {
@@ -698,6 +705,15 @@ DOOMS_CUDA_API int32_t dooms_cuda_matvec_split(int32_t dtype, const void * d_w, 
         (flags & ~(cuda::kFlagAccumulate | cuda::kFlagBias)) || (d_w2 && flags)) {
         return fail(DOOMS_INVALID_ARGUMENT, "matvec_split: NULL pointer, unknown flag, or rows that are not whole blocks");
     }
+    // the same choice of kernel as on an f32 input (matvec, gate_up), so that both give the same bits
+    if ((reinterpret_cast<uintptr_t>(d_split) & 15u) == 0 && cuda::gemv_short_supported(dtype, d_w, rows, cols, d_w2 ? 2 : 1) &&
+        (!d_w2 || cuda::gemv_short_supported(dtype, d_w2, rows, cols, 2))) {
+        const cuda::ShortMatrix m{dtype, d_w, d_w2, rows, d_y, d_bias};
+        return launch_result(cuda::launch_gemv_short(&m, 1, d_split, nullptr, nullptr, 0.f, cols, flags, static_cast<cudaStream_t>(stream)), "matvec_split");
+    }
+    if (!d_w2 && (reinterpret_cast<uintptr_t>(d_split) & 15u) == 0 && cuda::gemv_tall_supported(dtype, d_w, rows, cols)) {
+        return launch_result(cuda::launch_gemv_tall(dtype, d_w, d_split, nullptr, nullptr, 0.f, d_y, d_bias, rows, cols, flags, static_cast<cudaStream_t>(stream)), "matvec_split");
+    }
     const bool k4 = dtype == DOOMS_Q4_K;
     const bool ok = k4 ? cuda::gemv_q4_k_supported(d_w, rows, cols) && (!d_w2 || cuda::gemv_q4_k_supported(d_w2, rows, cols))
                        : cuda::gemv_q4_0_supported(d_w, rows, cols) && (!d_w2 || cuda::gemv_q4_0_supported(d_w2, rows, cols));
@@ -714,6 +730,10 @@ DOOMS_CUDA_API int32_t dooms_cuda_gate_up(int32_t dtype, const void * d_wg, cons
     }
     if (rows == 0) return DOOMS_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if ((reinterpret_cast<uintptr_t>(d_x) & 15u) == 0 && cuda::gemv_short_supported(dtype, d_wg, rows, cols, 2) && cuda::gemv_short_supported(dtype, d_wu, rows, cols, 2)) {
+        const cuda::ShortMatrix m{dtype, d_wg, d_wu, rows, d_h, nullptr};
+        return launch_result(cuda::launch_gemv_short(&m, 1, nullptr, d_x, nullptr, 0.f, cols, 0u, st), "gate_up");
+    }
     if (dtype == DOOMS_Q4_0 && cuda::gemv_q4_0_supported(d_wg, rows, cols) && cuda::gemv_q4_0_supported(d_wu, rows, cols)) {
         return fast_q4_0(d_wg, d_wu, d_x, d_h, nullptr, rows, cols, 0u, false, st, "gate_up");
     }

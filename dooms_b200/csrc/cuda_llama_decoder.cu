@@ -245,6 +245,32 @@ struct CudaLlamaDecoder::Impl {
     bool fast(const MatDev & w) const {
         return (w.dt == DType::Q4_0 && cuda::gemv_q4_0_supported(w.ptr, w.rows, w.cols)) || (w.dt == DType::Q4_K && cuda::gemv_q4_k_supported(w.ptr, w.rows, w.cols));
     }
+    // the kernel for small matrices takes all of these projections of one input (one launch)
+    static bool shortp(std::initializer_list<const MatDev *> ws, int nmat = 1, bool split_out = false) {
+        int64_t all = 0;
+        for (const MatDev * w : ws) all += w->rows;
+        for (const MatDev * w : ws) {
+            if (w->cols != (*ws.begin())->cols || (w->dt == DType::F16) != ((*ws.begin())->dt == DType::F16)) return false;
+            if (!cuda::gemv_short_supported(int(w->dt), w->ptr, w->rows, w->cols, nmat, split_out, nmat == 2 ? 0 : all)) return false;
+        }
+        return true;
+    }
+    static bool short_qkv(const LayerDev & L) {
+        if (L.qkv.size() == 1) return shortp({&L.qkv[0].w});
+        return L.qkv.size() == 3 && shortp({&L.qkv[0].w, &L.qkv[1].w, &L.qkv[2].w});
+    }
+    static bool short_gate_up(const LayerDev & L, bool split_out = false) {
+        return L.ffn_gate.dt == L.ffn_up.dt && shortp({&L.ffn_gate, &L.ffn_up}, 2, split_out);
+    }
+    // a projection that takes its input as a split row
+    bool takes_split(const MatDev & w) const {
+        return fast(w) || (w.dt != DType::F16 && shortp({&w})) || (w.dt == DType::Q6_K && cuda::gemv_q6_k_supported(w.ptr, w.rows, w.cols));
+    }
+    // a projection that takes its norm from the producer of its input (the wide shapes)
+    bool takes_link(const MatDev & w) const {
+        if (shortp({&w})) return w.dt != DType::F16 && !cuda::gemv_short_own_norm(w.cols);
+        return fast(w) || (w.dt != DType::F16 && cuda::gemv_tall_supported(int(w.dt), w.ptr, w.rows, w.cols));
+    }
     // One-token projection of `in`, RMS-normalized with gamma first when gamma is given. The streaming kernels do the norm (and the q4_0 kernel the split of
     // its input into int8 limbs) in their prologue; only shapes they do not take go through a norm launch and the row-per-warp kernel. A producer that
     // already wrote the split of `in` (the attention merge) leaves it in xq and says so in xq_of.
@@ -261,6 +287,24 @@ struct CudaLlamaDecoder::Impl {
     void matvec(const char * kind, const MatDev & w, const float * in, const float * gamma, float * out, const float * bias, uint32_t flags,
                 const float * next_gamma = nullptr) {
         const bool writes_x = out == x;
+        if (shortp({&w})) {
+            const cuda::ShortMatrix m{int(w.dt), w.ptr, nullptr, w.rows, out, bias};
+            const bool consume = gamma && in == x && link_ready && w.dt != DType::F16;
+            const void * split = w.dt == DType::F16 ? nullptr : consume ? xq2 : xq_of == in && !gamma ? xq : nullptr;
+            const cuda::GemvNormLink link{nullptr, nullptr, consume ? norm_ss : nullptr, consume ? link_blocks : 0};
+            run(kind, [&] { return cuda::launch_gemv_short(&m, 1, split, in, consume ? nullptr : gamma, cfg.rms_eps, w.cols, flags, stream, nullptr, &link); });
+            if (writes_x) link_ready = false;
+            return;
+        }
+        if (cuda::gemv_tall_supported(int(w.dt), w.ptr, w.rows, w.cols) && !writes_x) {
+            const bool consume = gamma && in == x && link_ready && w.dt != DType::F16;
+            const void * split = w.dt == DType::F16 ? nullptr : consume ? xq2 : (xq_of == in && !gamma) ? xq : nullptr;
+            const cuda::GemvNormLink link{nullptr, nullptr, consume ? norm_ss : nullptr, consume ? link_blocks : 0};
+            run(kind, [&] {
+                return cuda::launch_gemv_tall(int(w.dt), w.ptr, split, in, consume ? nullptr : gamma, cfg.rms_eps, out, bias, w.rows, w.cols, flags, stream, &link);
+            });
+            return;
+        }
         if (fast(w)) {
             const bool consume = gamma && in == x && link_ready;
             const bool produce = next_gamma && writes_x && tp == 1 && w.rows % 32 == 0 && norm_counters;
@@ -302,7 +346,21 @@ struct CudaLlamaDecoder::Impl {
         });
         xq_of = do_split ? xn : nullptr;
     }
-    void gate_up(const MatDev & wg, const MatDev & wu, const float * in, const float * gamma, float * out, bool down_takes_split) {
+    void gate_up(const LayerDev & L, const float * in, const float * gamma, float * out) {
+        const MatDev & wg = L.ffn_gate, & wu = L.ffn_up;
+        const bool down_takes_split = takes_split(L.ffn_down), half = wg.dt == DType::F16;
+        if (short_gate_up(L)) {
+            const bool split_out = down_takes_split && !half && short_gate_up(L, true);
+            const cuda::ShortMatrix m{int(wg.dt), wg.ptr, wu.ptr, wg.rows, out, nullptr};
+            const bool consume = gamma && in == x && link_ready && !half;
+            const void * split = half ? nullptr : consume ? xq2 : xq_of == in && !gamma ? xq : nullptr;
+            const cuda::GemvNormLink link{nullptr, nullptr, consume ? norm_ss : nullptr, consume ? link_blocks : 0};
+            run("gate_up", [&] {
+                return cuda::launch_gemv_short(&m, 1, split, in, consume ? nullptr : gamma, cfg.rms_eps, wg.cols, 0u, stream, split_out ? xq : nullptr, &link);
+            });
+            xq_of = split_out ? out : nullptr;
+            return;
+        }
         if (fast(wg) && fast(wu)) {
             const bool consume = gamma && in == x && link_ready;
             if (!consume) prepare_fast_input(in, gamma, wg.cols);
@@ -523,11 +581,25 @@ struct CudaLlamaDecoder::Impl {
             const bool use_tc = M > 1 && tc_capable && cfg.prefill_tile != 1;
             if (M > 1) norm(x, L.attn_norm, M, false, use_tc);
             if (M == 1) {
-                for (const QkvPart & q : L.qkv) {
-                    matvec("qkv", q.w, x, L.attn_norm, qkv + q.row0, L.qkv_bias ? L.qkv_bias + q.row0 : nullptr, L.qkv_bias ? kFlagBias : 0u);
+                if (short_qkv(L)) {      // one launch, also for parts of different types
+                    cuda::ShortMatrix parts[cuda::kShortParts];
+                    int n = 0;
+                    for (const QkvPart & q : L.qkv) {
+                        parts[n++] = cuda::ShortMatrix{int(q.w.dt), q.w.ptr, nullptr, q.w.rows, qkv + q.row0, L.qkv_bias ? L.qkv_bias + q.row0 : nullptr};
+                    }
+                    const bool consume = link_ready && L.qkv[0].w.dt != DType::F16;
+                    const cuda::GemvNormLink link{nullptr, nullptr, consume ? norm_ss : nullptr, consume ? link_blocks : 0};
+                    run("qkv", [&] {
+                        return cuda::launch_gemv_short(parts, n, consume ? xq2 : nullptr, x, consume ? nullptr : L.attn_norm, cfg.rms_eps, E, L.qkv_bias ? kFlagBias : 0u, stream,
+                                                       nullptr, &link);
+                    });
+                } else {
+                    for (const QkvPart & q : L.qkv) {
+                        matvec("qkv", q.w, x, L.attn_norm, qkv + q.row0, L.qkv_bias ? L.qkv_bias + q.row0 : nullptr, L.qkv_bias ? kFlagBias : 0u);
+                    }
                 }
                 // (a padded attention row is split by the projection itself: its zero columns are not the attention kernel's to write)
-                const bool split_attn = fast(L.attn_output) && cfg.head_dim % 32 == 0 && (gqa || splits > 1) && attn_width == q_width;
+                const bool split_attn = takes_split(L.attn_output) && cfg.head_dim % 32 == 0 && (gqa || splits > 1) && attn_width == q_width;
                 if (gqa) {
                     run("attention", [&] {
                         return cuda::launch_attention_gqa(qkv, kcl, vcl, part, state, inv_freq, 0, gqa_splits, as, attn_counters, attn + attn_pad, split_attn ? xq : nullptr, stream, rope_cs, cfg.n_ctx);
@@ -538,16 +610,16 @@ struct CudaLlamaDecoder::Impl {
                 }
                 xq_of = split_attn ? attn : nullptr;
                 // the projections that finish x also prepare the norm of the projection after them, when that one is a kernel that can take it
-                const bool gate_up_takes = fast(L.ffn_gate) && fast(L.ffn_up);
+                const bool gate_up_takes = short_gate_up(L) ? L.ffn_gate.dt != DType::F16 && !cuda::gemv_short_own_norm(E) : fast(L.ffn_gate) && fast(L.ffn_up);
                 matvec("attn_output", L.attn_output, attn, nullptr, o_dst, nullptr, o_flags, gate_up_takes ? L.ffn_norm : nullptr);
                 xq_of = nullptr;
                 reduce_into_x(1);
-                gate_up(L.ffn_gate, L.ffn_up, x, L.ffn_norm, h, fast(L.ffn_down));
+                gate_up(L, x, L.ffn_norm, h);
                 const float * after_gamma = nullptr;
                 if (l + 1 < layers.size()) {
                     const LayerDev & N = layers[l + 1];
-                    if (std::all_of(N.qkv.begin(), N.qkv.end(), [&](const QkvPart & q) { return fast(q.w); })) after_gamma = N.attn_norm;
-                } else if (output.rows > 0 && fast(output)) {
+                    if (std::all_of(N.qkv.begin(), N.qkv.end(), [&](const QkvPart & q) { return takes_link(q.w); })) after_gamma = N.attn_norm;
+                } else if (output.rows > 0 && takes_link(output)) {
                     after_gamma = output_norm;
                 }
                 matvec("ffn_down", L.ffn_down, h, nullptr, o_dst, nullptr, o_flags, after_gamma);

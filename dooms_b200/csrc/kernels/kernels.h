@@ -133,6 +133,18 @@ cudaError_t launch_argmax_pairs(const void * pairs, int n_ranks, int32_t * token
 // The same reduction without a state: *out = argmax.
 cudaError_t launch_argmax_plain(const float * logits, int64_t n, int32_t * out, void * part, cudaStream_t stream);
 
+// ---- the decode GEMV for small matrices (gemv_short.cu) ----
+// Takes f16, q4_0, q5_0 and q8_0 rows of whole pairs of blocks (16-byte aligned base) whose share per SM fits beside other kernels' blocks. all_rows: the rows
+// of all matrices of the launch (0: this one alone); nmat 2: a gate / up pair; split_out: the results are to be left split as well (rows a multiple of 32).
+constexpr int kShortParts = 3;
+struct ShortMatrix { int dt; const void * W; const void * W2; int64_t rows; float * y; const float * bias; };
+bool gemv_short_supported(int dt, const void * W, int64_t rows, int64_t cols, int nmat, bool split_out = false, int64_t all_rows = 0);
+// y (+)= W x (+ bias) for up to kShortParts matrices on one input, or (one entry with W2) y = silu(W x) * (W2 x). The input as for launch_gemv_q4_0: split (xq;
+// block formats only), or f32 x, normalized first when gamma is given. All entries are f16 or none is. xq_out (one entry): y split for the next projection.
+cudaError_t launch_gemv_short(const ShortMatrix * mats, int n, const void * xq, const float * x, const float * gamma, float eps, int64_t cols, uint32_t flags,
+                              cudaStream_t stream, void * xq_out = nullptr, const struct GemvNormLink * link = nullptr);      // link: as consumer only
+bool gemv_short_own_norm(int64_t cols);      // rows of this length are best normalized by the kernel itself; wider ones by their producer (GemvNormLink)
+
 // ---- the fast decode GEMV on q4_0 rows (gemv_q4_0.cu) ----
 // q6_K rows on the int8 tensor-core path (gemv_q6_k.cu): y (+)= W x (+ bias) on an input that is already split (launch_quantize_x, or a norm that leaves
 // the split). Takes 16-byte aligned matrices with rows of whole super-blocks, up to 40960 columns.
@@ -163,6 +175,10 @@ bool gemv_q4_k_supported(const void * W, int64_t rows, int64_t cols);
 // the producer's ss_out and its block count; the results are multiplied by rsqrt(sum(ss_in) / cols + eps), which is the norm's scale factor applied
 // after the product instead of before it.
 struct GemvNormLink { const float * gamma_out; float * ss_out; const float * ss_in; int ss_n; };
+// The GEMV for tall matrices (gemv_short.cu): the formats, inputs and flags of launch_gemv_short; link: as consumer only.
+bool gemv_tall_supported(int dt, const void * W, int64_t rows, int64_t cols);
+cudaError_t launch_gemv_tall(int dt, const void * W, const void * xq, const float * x, const float * gamma, float eps, float * y, const float * bias, int64_t rows, int64_t cols,
+                             uint32_t flags, cudaStream_t stream, const GemvNormLink * link = nullptr);
 int gemv_q4_0_blocks(int64_t rows, int64_t cols, bool gate_up, bool q4_k);      // blocks a launch on this shape uses
 cudaError_t launch_gemv_q4_0(const void * W, const void * W2, const void * xq, const float * x, const float * gamma, float eps, float * y, const float * bias,
                              int64_t rows, int64_t cols, uint32_t flags, bool q4_k, cudaStream_t stream, void * xq_out = nullptr, int * out_counters = nullptr,

@@ -10,10 +10,8 @@ namespace dev {
 
 // One warp, one block: lane holds element `lane` of block blk.
 __device__ __forceinline__ void split_block(float v, int lane, int blk, int nb, uint8_t * xq) {
-    float amax = fabsf(v);
-    #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    uint32_t eb = (__float_as_uint(amax) >> 23) & 0xFFu;       // biased exponent of the largest magnitude
+    const uint32_t amax = __reduce_max_sync(0xffffffffu, __float_as_uint(v) & 0x7FFFFFFFu);      // magnitudes order like their bits, infinities and NaN on top
+    uint32_t eb = amax >> 23;                                  // biased exponent of the largest magnitude
     eb = max(eb, 30u);                                         // blocks below 2^-97 are treated as that small: their digits come out zero
     eb = min(eb, 250u);
     const float inv = __uint_as_float((279u - eb) << 23);      // 2^26 / s with s = 2^(eb - 126) > amax
@@ -28,8 +26,9 @@ __device__ __forceinline__ void split_block(float v, int lane, int blk, int nb, 
     for (int i = 0; i < 4; i++) dst[i * 32 + pos] = uint8_t(int8_t(l[i]));
     if (lane == 0) {
         float * sx = reinterpret_cast<float *>(xq + size_t(nb) * 128) + blk * 2;
-        sx[0] = __uint_as_float((eb - 29u) << 23);             // s * 2^-26 / 16: the weights carry a factor 16
-        sx[1] = __uint_as_float((eb - 15u) << 23);             // the same for the upper digit pair (x 2^14)
+        const bool finite = amax < 0x7F800000u;                // a block with an infinity or a NaN in it makes every sum it enters NaN
+        sx[0] = __uint_as_float(finite ? (eb - 29u) << 23 : 0x7FC00000u);      // s * 2^-26 / 16: the weights carry a factor 16
+        sx[1] = __uint_as_float(finite ? (eb - 15u) << 23 : 0x7FC00000u);      // the same for the upper digit pair (x 2^14)
     }
 }
 
