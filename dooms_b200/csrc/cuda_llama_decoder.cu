@@ -110,7 +110,9 @@ struct CudaLlamaDecoder::Impl {
     int splits = 1;
     static constexpr int kMaxShares = 32;
     __half * rows16_all = nullptr;   // batched decode steps: the matrices as f16 rows (MatDev::rows16 point into it), when memory allows
-    float * b_shares = nullptr;  // batched decode steps: [share][max_rows][n_embd] sums of the blocks that share a tile's reduction
+    float * shares = nullptr;    // [share][row][n_embd] sums of the blocks that share a tile's reduction (gemm_into_x)
+    size_t share_floats = 0;
+    int pending_shares = 0;      // that many of them are still to be added onto x
     bool rows_tc = false;        // batched decode steps: attention on the tensor cores (attention_rows.cu)
     bool gqa = false;            // decode attention: the grouped-query kernel (which also rotates and stores the new key / value)
     int gqa_splits = 1;
@@ -171,7 +173,7 @@ struct CudaLlamaDecoder::Impl {
         if (step_graph) cudaGraphExecDestroy(step_graph);      // a graph that holds captured NCCL work has to go before its communicator
         cuda::decode_layers_destroy(fused);
         for (auto & g : batch_graphs) cudaGraphExecDestroy(g.second);
-        for (void * p : {(void *)b_rows, (void *)b_out, (void *)b_step, (void *)b_logits, (void *)b_part, b_argmax_part, (void *)b_counters, (void *)b_shares, (void *)rows16_all}) if (p) cudaFree(p);
+        for (void * p : {(void *)b_rows, (void *)b_out, (void *)b_step, (void *)b_logits, (void *)b_part, b_argmax_part, (void *)b_counters, (void *)shares, (void *)rows16_all}) if (p) cudaFree(p);
         for (void * p : {(void *)h_rows, (void *)h_out}) if (p) cudaFreeHost(p);
         for (void * p : par_opened) cudaIpcCloseMemHandle(p);
         for (void * p : {par_inbox, par_flags, par_words}) if (p) cudaFree(p);
@@ -341,9 +343,12 @@ struct CudaLlamaDecoder::Impl {
     // input invalidates the split copy).
     void norm(const float * in, const float * gamma, int M, bool split, bool f16_only = false) {
         const bool do_split = split && M == 1 && cfg.n_embd % 32 == 0;
+        const int n_shares = in == x ? pending_shares : 0;
         run("norm", [&] {
-            return cuda::launch_rms_norm(in, gamma, f16_only ? nullptr : xn, f16_only ? xn16 : nullptr, do_split ? xq : nullptr, M, cfg.n_embd, cfg.rms_eps, stream);
+            return cuda::launch_rms_norm(in, gamma, f16_only ? nullptr : xn, f16_only ? xn16 : nullptr, do_split ? xq : nullptr, M, cfg.n_embd, cfg.rms_eps, stream,
+                                         shares, n_shares, int64_t(M) * cfg.n_embd);
         });
+        if (in == x) pending_shares = 0;
         xq_of = do_split ? xn : nullptr;
     }
     void gate_up(const LayerDev & L, const float * in, const float * gamma, float * out) {
@@ -406,6 +411,7 @@ struct CudaLlamaDecoder::Impl {
     }
     // Starts writing the f16 rows of w into the next of the two buffers, on the second stream, as soon as the product that last read that buffer is done.
     int rows_prefetch(const MatDev & w) {
+        if (w.rows16) return -1;
         const int s = rows_next;
         rows_next ^= 1;
         cudaStreamWaitEvent(side, rows_freed[s], 0);
@@ -413,28 +419,44 @@ struct CudaLlamaDecoder::Impl {
         cudaEventRecord(rows_filled[s], side);
         return s;
     }
+    // A projection of a chunk: on the rows that rows_prefetch put into buffer slot (slot >= 0), on the decoder's own f16 copy, or as launch_gemm_tc decides.
+    void gemm_chunk(const char * kind, const MatDev & w, int slot, const cuda::TensorMap & map, float * out, const float * bias, int M, int64_t out_stride, uint32_t flags) {
+        if (slot >= 0) gemm_from_rows(kind, w, slot, map, out, bias, M, out_stride, flags);
+        else gemm_rows(kind, w, nullptr, map, out, nullptr, bias, M, out_stride, 0, flags);
+    }
     // The product on the rows that rows_prefetch put into buffer s.
     void gemm_from_rows(const char * kind, const MatDev & w, int s, const cuda::TensorMap & map, float * out, const float * bias, int M, int64_t out_stride, uint32_t flags) {
         cudaStreamWaitEvent(stream, rows_filled[s], 0);
         run(kind, [&] { return cuda::launch_gemm_tc_rows16(rows_buf[s], nullptr, &map, out, nullptr, bias, M, w.rows, w.cols, out_stride, 0, flags, host_error, stream); });
         cudaEventRecord(rows_freed[s], stream);
     }
-    // x[m] += X16[m] . W[n] for the rows of a batched step. Few weight rows against one token tile would run on a handful of SMs, so the reduction
-    // dimension is dealt over several blocks per tile where that pays; their sums are added onto x in a fixed order.
-    void gemm_tc_into_x(const char * kind, const MatDev & w, const cuda::TensorMap & map, int M) {
+    // x[m] += X16[m] . W[n] for the rows of a chunk or of a batched step. Few weight rows against few token tiles would run on a handful of SMs, so the reduction
+    // dimension is dealt over several blocks per tile where that pays; their sums stay in `shares` (pending_shares of them), and the norm that reads x next
+    // adds them onto it in a fixed order. slot >= 0: the matrix's f16 rows are in rows_buf[slot].
+    void gemm_into_x(const char * kind, const MatDev & w, int slot, const cuda::TensorMap & map, int M, float * dst, uint32_t flags) {
         const int E = cfg.n_embd;
-        int shares = 1;
-        if (b_shares) shares = w.rows16 ? cuda::gemm_tc_rows16_k_splits(M, w.rows, w.cols) : cuda::gemm_tc_k_splits(int(w.dt), M, w.rows, w.cols, false, w16 ? w16_bytes : 0);
-        if (shares <= 1 || shares > kMaxShares) { gemm_rows(kind, w, nullptr, map, x, nullptr, nullptr, M, E, 0, kFlagAccumulate); return; }
-        const int64_t share_stride = int64_t(max_rows) * E;
+        const int64_t share_stride = int64_t(M) * E;
+        const int most = tp == 1 && shares ? int(std::min<int64_t>(kMaxShares, int64_t(share_floats) / share_stride)) : 1;
+        const __half * rows = slot >= 0 ? rows_buf[slot] : w.rows16;
+        const int n = most < 2 ? 1 : rows ? cuda::gemm_tc_rows16_k_splits(M, w.rows, w.cols, most)
+                                          : cuda::gemm_tc_k_splits(int(w.dt), w.ptr, M, w.rows, w.cols, w16 ? w16_bytes : 0, most);
+        float * out = n > 1 ? shares : dst;
+        const uint32_t f = n > 1 ? 0u : flags;
+        if (slot >= 0) cudaStreamWaitEvent(stream, rows_filled[slot], 0);
         run(kind, [&] {
-            if (w.rows16) {
-                return cuda::launch_gemm_tc_rows16(w.rows16, nullptr, &map, b_shares, nullptr, nullptr, M, w.rows, w.cols, E, 0, 0u, host_error, stream, shares, share_stride);
-            }
-            return cuda::launch_gemm_tc(int(w.dt), w.ptr, nullptr, &map, b_shares, nullptr, nullptr, M, w.rows, w.cols, E, 0, 0u, host_error, stream, w16, w16_bytes, shares,
-                                        share_stride);
+            if (rows) return cuda::launch_gemm_tc_rows16(rows, nullptr, &map, out, nullptr, nullptr, M, w.rows, w.cols, E, 0, f, host_error, stream, n, share_stride);
+            return cuda::launch_gemm_tc(int(w.dt), w.ptr, nullptr, &map, out, nullptr, nullptr, M, w.rows, w.cols, E, 0, f, host_error, stream, w16, w16_bytes, n, share_stride);
         });
-        run("residual", [&] { return cuda::launch_add_shares(x, b_shares, shares, int64_t(M) * E, share_stride, stream); });
+        if (slot >= 0) cudaEventRecord(rows_freed[slot], stream);
+        pending_shares = n > 1 ? n : 0;
+        if (n == 1) reduce_into_x(M);
+    }
+    // The same for a caller that reads row m of x itself.
+    void finish_row(int m, int M) {
+        if (pending_shares == 0) return;
+        const int64_t E = cfg.n_embd;
+        run("residual", [&] { return cuda::launch_add_shares(x + m * E, shares + m * E, pending_shares, E, int64_t(M) * E, stream); });
+        pending_shares = 0;
     }
     // A projection of a batched step: from the decoder's f16 copy of the matrix when it keeps one, else as any chunk's.
     void gemm_rows(const char * kind, const MatDev & w, const MatDev * w2, const cuda::TensorMap & map, float * out, __half * out16, const float * bias, int M,
@@ -624,35 +646,24 @@ struct CudaLlamaDecoder::Impl {
                 }
                 matvec("ffn_down", L.ffn_down, h, nullptr, o_dst, nullptr, o_flags, after_gamma);
                 reduce_into_x(1);
-            } else if (use_tc && rows_ahead && M >= 128 && !profile) {
-                // (the chunk's norm above wrote xn16) Every projection but the fused gate / up reads f16 rows that were written while the kernels before
-                // it ran: the rows of attn_output during the qkv product, those of ffn_down during attention, the next layer's qkv during gate / up.
-                if (l == 0) rows_slot = rows_prefetch(L.qkv[0].w);
-                const int slot_qkv = rows_slot, slot_o = rows_prefetch(L.attn_output);
-                gemm_from_rows("qkv", L.qkv[0].w, slot_qkv, map_xn, qkv, L.qkv_bias, M, qkv_width, L.qkv_bias ? kFlagBias : 0u);
-                run("rope_store", [&] { return cuda::launch_rope_store(qkv, kcl, vcl, state, inv_freq, M, as, stream); });
-                prefill_attention(kcl, vcl, attn16, M, as);
-                const int slot_down = rows_prefetch(L.ffn_down);
-                gemm_from_rows("attn_output", L.attn_output, slot_o, map_attn, o_dst, nullptr, M, E, o_flags);
-                reduce_into_x(M);
-                norm(x, L.ffn_norm, M, false, true);
-                gemm_tc("gate_up", L.ffn_gate, &L.ffn_up, map_xn, nullptr, h16, nullptr, M, 0, ff, 0u);
-                if (l + 1 < layers.size()) rows_slot = rows_prefetch(layers[l + 1].qkv[0].w);
-                gemm_from_rows("ffn_down", L.ffn_down, slot_down, map_h, o_dst, nullptr, M, E, o_flags);
-                reduce_into_x(M);
             } else if (use_tc) {
-                // (the chunk's norm above wrote xn16)
+                // (the chunk's norm above wrote xn16) From 128 tokens on, every projection but the fused gate / up reads f16 rows that were written while the
+                // kernels before it ran: the rows of attn_output during the qkv product, those of ffn_down during attention, the next layer's qkv during
+                // gate / up. A decoder that keeps f16 copies of its matrices (batched steps) reads those instead.
+                const bool ahead = rows_ahead && M >= 128 && !profile;
+                if (ahead && l == 0) rows_slot = rows_prefetch(L.qkv[0].w);
+                const int slot_qkv = ahead ? rows_slot : -1, slot_o = ahead ? rows_prefetch(L.attn_output) : -1;
                 for (const QkvPart & q : L.qkv) {
-                    gemm_tc("qkv", q.w, nullptr, map_xn, qkv + q.row0, nullptr, L.qkv_bias ? L.qkv_bias + q.row0 : nullptr, M, qkv_width, 0, L.qkv_bias ? kFlagBias : 0u);
+                    gemm_chunk("qkv", q.w, slot_qkv, map_xn, qkv + q.row0, L.qkv_bias ? L.qkv_bias + q.row0 : nullptr, M, qkv_width, L.qkv_bias ? kFlagBias : 0u);
                 }
                 run("rope_store", [&] { return cuda::launch_rope_store(qkv, kcl, vcl, state, inv_freq, M, as, stream); });
                 prefill_attention(kcl, vcl, attn16, M, as);
-                gemm_tc("attn_output", L.attn_output, nullptr, map_attn, o_dst, nullptr, nullptr, M, E, 0, o_flags);
-                reduce_into_x(M);
+                const int slot_down = ahead ? rows_prefetch(L.ffn_down) : -1;
+                gemm_into_x("attn_output", L.attn_output, slot_o, map_attn, M, o_dst, o_flags);
                 norm(x, L.ffn_norm, M, false, true);
-                gemm_tc("gate_up", L.ffn_gate, &L.ffn_up, map_xn, nullptr, h16, nullptr, M, 0, ff, 0u);
-                gemm_tc("ffn_down", L.ffn_down, nullptr, map_h, o_dst, nullptr, nullptr, M, E, 0, o_flags);
-                reduce_into_x(M);
+                gemm_rows("gate_up", L.ffn_gate, &L.ffn_up, map_xn, nullptr, h16, nullptr, M, 0, ff, 0u);
+                if (ahead && l + 1 < layers.size()) rows_slot = rows_prefetch(layers[l + 1].qkv[0].w);
+                gemm_into_x("ffn_down", L.ffn_down, slot_down, map_h, M, o_dst, o_flags);
             } else {
                 for (const QkvPart & q : L.qkv) {
                     matmul("qkv", q.w, nullptr, xn, E, qkv + q.row0, qkv_width, L.qkv_bias ? L.qkv_bias + q.row0 : nullptr, M, L.qkv_bias ? kFlagBias : 0u);
@@ -667,6 +678,7 @@ struct CudaLlamaDecoder::Impl {
                 reduce_into_x(M);
             }
         }
+        finish_row(M - 1, M);
         // The logits of the last row only (metal_llama_decoder.mm:375).
         if (output.rows > 0) matvec("output", output, x + size_t(M - 1) * E, output_norm, logits_buf + vocab_row0, nullptr, 0u);
         if (tp > 1) {
@@ -747,10 +759,10 @@ struct CudaLlamaDecoder::Impl {
                 return cuda::launch_attention_gqa_rows(qkv, kc + l * cache_layer_elems, vc + l * cache_layer_elems, b_part, inv_freq, b_splits, as, b_counters, attn, attn16,
                                                        rows, n, stream);
             });
-            gemm_tc_into_x("attn_output", L.attn_output, map_attn, n);
+            gemm_into_x("attn_output", L.attn_output, -1, map_attn, n, x, kFlagAccumulate);
             norm(x, L.ffn_norm, n, false, true);
             gemm_rows("gate_up", L.ffn_gate, &L.ffn_up, map_xn, nullptr, h16, nullptr, n, 0, ff, 0u);
-            gemm_tc_into_x("ffn_down", L.ffn_down, map_h, n);
+            gemm_into_x("ffn_down", L.ffn_down, -1, map_h, n, x, kFlagAccumulate);
         }
         norm(x, output_norm, n, false, true);
         gemm_rows("output", output, nullptr, map_xn, b_logits, nullptr, nullptr, n, cfg.n_vocab, 0, 0u);
@@ -1150,6 +1162,15 @@ Result<std::unique_ptr<CudaLlamaDecoder>> CudaLlamaDecoder::create(const LlamaDe
     // a decode step over several slots needs the tensor-core chunk path, the grouped-query attention kernel and the whole model on this GPU
     m.max_rows = (n_seq > 1 && tp == 1 && m.tc_capable && m.gqa && cuda::gemm_tc_supported(int(m.output.dt), m.output.ptr, m.output.rows, m.output.cols))
                      ? std::min<int32_t>({n_seq, c.n_batch, 1024}) : 0;
+    if (m.tc_capable && tp == 1) {
+        // room for the shares of a reduction: what a batched step may want, at least 24 MB (ten shares of a 512-token chunk of 896-wide rows, eleven of a
+        // 128-token one of 4096); optional, without it no product is dealt
+        m.share_floats = std::max<size_t>(size_t(6) << 20, size_t(Impl::kMaxShares) * size_t(m.max_rows) * size_t(E));
+        if (cudaMalloc(reinterpret_cast<void **>(&m.shares), m.share_floats * sizeof(float)) != cudaSuccess) {
+            (void)cudaGetLastError();
+            m.shares = nullptr;
+        }
+    }
     if (m.max_rows > 0) {
         const size_t R = size_t(m.max_rows);
         // Rows attend over very different lengths (a fresh sequence beside one at the end of its context), so a row is cut into ranges of a fixed number of
@@ -1164,10 +1185,6 @@ Result<std::unique_ptr<CudaLlamaDecoder>> CudaLlamaDecoder::create(const LlamaDe
         DOOMS_RETURN_IF_ERROR(dev_alloc(reinterpret_cast<void **>(&m.b_part), R * size_t(m.b_splits) * size_t(m.nh) * size_t(2 + c.head_dim) * sizeof(float), "the batched attention partial results"));
         DOOMS_RETURN_IF_ERROR(dev_alloc(&m.b_argmax_part, R * size_t(cuda::argmax_blocks(c.n_vocab)) * 8, "the batched argmax partial results"));
         DOOMS_RETURN_IF_ERROR(dev_alloc(reinterpret_cast<void **>(&m.b_counters), R * size_t(m.nkv) * sizeof(int), "the batched attention counters"));
-        if (cudaMalloc(reinterpret_cast<void **>(&m.b_shares), size_t(Impl::kMaxShares) * R * size_t(E) * sizeof(float)) != cudaSuccess) {      // optional
-            (void)cudaGetLastError();
-            m.b_shares = nullptr;
-        }
         // Batched steps run every projection from f16 rows. A copy of the matrices in that form, made once, saves dequantizing them in every step (11 % of
         // a 256-row step on the 0.5B shape); it is kept when it takes at most a quarter of the memory that is still free (DOOMS_BATCH_F16_ROWS=0: never).
         std::vector<MatDev *> mats;

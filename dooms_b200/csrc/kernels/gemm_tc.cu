@@ -43,6 +43,7 @@ constexpr int kStepK = 64;          // k elements per stage: one 128-byte swizzl
 constexpr int kProducerWarps = 8;   // two threads per weight row
 constexpr int kThreads = (kProducerWarps + 2) * 32;   // + the TMA warp and the MMA warp
 constexpr uint32_t kTileWBytes = kRowsW * kStepK * 2; // 16 KB
+constexpr int kTokenBox = 64;       // token rows per tensor copy (and the smallest token tile)
 
 // ---- tcgen05 / TMA wrappers ----
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap * map, int x, int y, uint32_t bar) {
@@ -205,7 +206,7 @@ struct GemmTcParams {
     int K, M;                  // reduction length, tokens
     int64_t y_stride, y16_stride;
     uint32_t flags;
-    int T;                     // tokens per block: 128 or 256
+    int T;                     // tokens per block: 64, 128 or 256 (an accumulator takes T columns of tensor memory)
     int wide;                  // q4_0 / q4_K rows of whole 256-element groups at 16-byte aligned addresses: the producers load 144-byte groups with 16-byte loads
     int pair;                  // (the two-matrix kernel) the second matrix is the next 128 rows of W: one block computes 256 weight rows against its token tile
     int ks_per;                // k steps per block along gridDim.z (0: all of them, one block per tile); block z writes its sum to Y + z * split_stride
@@ -219,11 +220,10 @@ struct GemmTcParams {
 // PRE: the weights were dequantized to f16 rows beforehand (k_dequant_f16; the reference's dequant_half + matmul_big pair for large M,
 // llama_kernels.h:1474-1480, metal_llama_decoder.mm:31): their tiles arrive by TMA like the token tile (wmap / w2map), the producer warps only run the
 // epilogue, and the stage's single "full" barrier counts the bytes of all its tiles.
-template <int DT, bool GATE, bool PRE>
+template <int DT, bool GATE, bool PRE, int STAGES>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                                                          const __grid_constant__ CUtensorMap w2map, const GemmTcParams p) {
     constexpr int NMAT = GATE ? 2 : 1;
-    constexpr int STAGES = GATE ? 3 : 4;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t tile_x_bytes = uint32_t(p.T) * 128u;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
     // a share of the reduction (f16-row path only): k steps ks0 .. ks0 + ksteps - 1
     const int ks0 = p.ks_per > 0 ? int(blockIdx.z) * p.ks_per : 0;
     const int ksteps = p.ks_per > 0 ? min(p.K / kStepK - ks0, p.ks_per) : p.K / kStepK;
-    const uint32_t ncols = GATE ? 512u : 256u;
+    const uint32_t ncols = uint32_t(p.T) * NMAT;      // the second accumulator starts T columns behind the first
 
     if (!(p.flags & kFlagLateDependents)) pdl_trigger();
     if (threadIdx.x == 0) {
@@ -352,7 +352,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
                 if (!ok) break;
                 const uint32_t dst = smem0 + s * stage_bytes + NMAT * kTileWBytes;
                 mbar_arrive_expect_tx(full_x + 8 * s, tile_x_bytes + (PRE ? NMAT * kTileWBytes : 0u));
-                for (int part = 0; part < p.T / 128; part++) tma_load_2d(dst + part * 16384u, &xmap, (ks0 + ks) * kStepK, m0 + part * 128, full_x + 8 * s);
+                for (int part = 0; part < p.T / kTokenBox; part++) {
+                    tma_load_2d(dst + part * (kTokenBox * 128u), &xmap, (ks0 + ks) * kStepK, m0 + part * kTokenBox, full_x + 8 * s);
+                }
                 if (PRE) {
                     tma_load_2d(smem0 + s * stage_bytes, &wmap, (ks0 + ks) * kStepK, int(n0), full_x + 8 * s);
                     if (GATE) tma_load_2d(smem0 + s * stage_bytes + kTileWBytes, &w2map, (ks0 + ks) * kStepK, int(n0) + (pair ? kRowsW : 0), full_x + 8 * s);
@@ -381,7 +383,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
                     const uint64_t bdesc = smem_desc_sw128(xt + kk * 32);
                     #pragma unroll
                     for (int mtx = 0; mtx < NMAT; mtx++) {
-                        tc_mma_f16(tmem_base + mtx * 256u, smem_desc_sw128(wt + mtx * kTileWBytes + kk * 32), bdesc, idesc, (ks | kk) ? 1u : 0u);
+                        tc_mma_f16(tmem_base + mtx * uint32_t(p.T), smem_desc_sw128(wt + mtx * kTileWBytes + kk * 32), bdesc, idesc, (ks | kk) ? 1u : 0u);
                     }
                 }
                 tc_commit(empty + 8 * s);      // arrives when the MMAs above have read the stage
@@ -408,7 +410,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
                     uint32_t acc[32], acc2[32];
                     const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(c0);
                     tc_ld32(taddr, acc);
-                    tc_ld32(taddr + 256u, acc2);
+                    tc_ld32(taddr + uint32_t(p.T), acc2);
                     #pragma unroll
                     for (int j = 0; j < 32; j++) {
                         dst[int64_t(c0 + j) * kRowsW] = __uint_as_float(acc[j]);
@@ -420,30 +422,49 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
             for (int part = 0; part < (pair ? 2 : 1); part++) {
                 const int64_t n = n0 + part * kRowsW + q * 32 + lane;
                 const float bias = (p.flags & kFlagBias) && n < p.N ? p.bias[n] : 0.f;
+                // Per result the code has to stay at a handful of instructions (pointers that step by a row, conditions outside the loops): 32768 of them pass
+                // through a tile's eight warps, and at the 52 instructions each that index arithmetic and conditions per element took, a 512-token product
+                // of 896 x 1152 spent 13 of its 22 us here.
+                const bool adds = Y && (p.flags & kFlagAccumulate);
                 for (int c0 = colhalf * cols_per_warp; c0 < (colhalf + 1) * cols_per_warp; c0 += 32) {
                     if (m0 + c0 >= p.M) break;      // warp-uniform
+                    const int limit = n < p.N ? min(32, p.M - (m0 + c0)) : 0;      // this lane's results to write
                     uint32_t acc[32], acc2[32];
-                    const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(c0) + uint32_t(part) * 256u;
+                    const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(c0) + uint32_t(part * p.T);
+                    float * const y0 = Y + int64_t(m0 + c0) * p.y_stride + n;
                     // what the results are added to: all 32 loads of a lane are asked for before the first is used (one after another, each behind the
                     // store before it, they cost a memory latency apiece: 4 x 32 of them per tile)
                     float old[32];
-                    const bool adds = Y && (p.flags & kFlagAccumulate) && n < p.N;
-                    #pragma unroll
-                    for (int j = 0; j < 32; j++) old[j] = (adds && m0 + c0 + j < p.M) ? __ldcg(Y + int64_t(m0 + c0 + j) * p.y_stride + n) : 0.f;
+                    if (adds) {
+                        const float * o = y0;
+                        #pragma unroll
+                        for (int j = 0; j < 32; j++) { old[j] = j < limit ? __ldcg(o) : 0.f; o += p.y_stride; }
+                    }
                     tc_ld32(taddr, acc);
-                    if (GATE && !pair) tc_ld32(taddr + 256u, acc2);
-                    if (n < p.N) {
+                    if (GATE && !pair) {
+                        tc_ld32(taddr + uint32_t(p.T), acc2);
                         #pragma unroll
                         for (int j = 0; j < 32; j++) {
-                            const int m = m0 + c0 + j;
-                            if (m >= p.M) continue;
-                            float v = __uint_as_float(acc[j]);
-                            if (GATE && !pair) v = v / (1.f + expf(-v)) * __uint_as_float(acc2[j]);
-                            else v += bias;
-                            v += old[j];
-                            if (Y) Y[int64_t(m) * p.y_stride + n] = v;
-                            if (p.Y16) p.Y16[int64_t(m) * p.y16_stride + n] = __float2half_rn(v);
+                            const float v = __uint_as_float(acc[j]);
+                            acc[j] = __float_as_uint(v / (1.f + expf(-v)) * __uint_as_float(acc2[j]));
                         }
+                    } else {
+                        #pragma unroll
+                        for (int j = 0; j < 32; j++) acc[j] = __float_as_uint(__uint_as_float(acc[j]) + bias);
+                    }
+                    if (adds) {
+                        #pragma unroll
+                        for (int j = 0; j < 32; j++) acc[j] = __float_as_uint(__uint_as_float(acc[j]) + old[j]);
+                    }
+                    if (Y) {
+                        float * o = y0;
+                        #pragma unroll
+                        for (int j = 0; j < 32; j++) { if (j < limit) *o = __uint_as_float(acc[j]); o += p.y_stride; }
+                    }
+                    if (p.Y16) {
+                        __half * o = p.Y16 + int64_t(m0 + c0) * p.y16_stride + n;
+                        #pragma unroll
+                        for (int j = 0; j < 32; j++) { if (j < limit) *o = __float2half_rn(__uint_as_float(acc[j])); o += p.y16_stride; }
                     }
                 }
             }
@@ -471,18 +492,33 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-template <int DT, bool PRE>
-cudaError_t launch_tiles(const CUtensorMap & map, const CUtensorMap & wmap, const CUtensorMap & w2map, const GemmTcParams & p, bool gate, int n_tiles, cudaStream_t stream) {
-    const size_t stage = (gate ? 2 : 1) * size_t(kTileWBytes) + size_t(p.T) * 128;
-    const size_t smem = (gate ? 3 : 4) * stage + 1024 + 256;
+template <int DT, bool GATE, bool PRE, int STAGES>
+cudaError_t launch_staged(const CUtensorMap & map, const CUtensorMap & wmap, const CUtensorMap & w2map, const GemmTcParams & p, int n_tiles, cudaStream_t stream) {
+    const size_t stage = (GATE ? 2 : 1) * size_t(kTileWBytes) + size_t(p.T) * 128;
+    const size_t smem = STAGES * stage + 1024 + 512;
     const int k_blocks = p.ks_per > 0 ? (p.K / kStepK + p.ks_per - 1) / p.ks_per : 1;
     const dim3 grid(unsigned(n_tiles), 1u, unsigned(k_blocks));
-    static std::atomic<uint64_t> configured[2];
-    if (const cudaError_t e = gate ? allow_dynamic_smem(k_gemm_tc<DT, true, PRE>, 220 * 1024, configured[1])
-                                   : allow_dynamic_smem(k_gemm_tc<DT, false, PRE>, 220 * 1024, configured[0]); e != cudaSuccess) return e;
+    static std::atomic<uint64_t> configured{0};
+    if (const cudaError_t e = allow_dynamic_smem(k_gemm_tc<DT, GATE, PRE, STAGES>, 220 * 1024, configured); e != cudaSuccess) return e;
     // launched early: the block's set-up (mbarriers, tensor memory) overlaps the end of the kernel before it
-    if (gate) return launch_pdl(k_gemm_tc<DT, true, PRE>, grid, dim3(kThreads), smem, stream, map, wmap, w2map, p);
-    return launch_pdl(k_gemm_tc<DT, false, PRE>, grid, dim3(kThreads), smem, stream, map, wmap, w2map, p);
+    return launch_pdl(k_gemm_tc<DT, GATE, PRE, STAGES>, grid, dim3(kThreads), smem, stream, map, wmap, w2map, p);
+}
+// Stages: what fits 200 KB on the f16-row path (24, 32 or 48 KB a stage; 40, 48 or 64 KB with two weight tiles): a product of few tiles waits for its copies, not
+// for the tensor core, so the bytes in flight per SM are its speed. The producers' path keeps the depth its threads' step counting was laid out for.
+template <int DT, bool PRE>
+cudaError_t launch_tiles(const CUtensorMap & map, const CUtensorMap & wmap, const CUtensorMap & w2map, const GemmTcParams & p, bool gate, int n_tiles, cudaStream_t stream) {
+    if constexpr (PRE) {
+        if (gate) {
+            if (p.T == 64) return launch_staged<DT, true, true, 5>(map, wmap, w2map, p, n_tiles, stream);
+            if (p.T == 128) return launch_staged<DT, true, true, 4>(map, wmap, w2map, p, n_tiles, stream);
+            return launch_staged<DT, true, true, 3>(map, wmap, w2map, p, n_tiles, stream);
+        }
+        if (p.T == 64) return launch_staged<DT, false, true, 8>(map, wmap, w2map, p, n_tiles, stream);
+        if (p.T == 128) return launch_staged<DT, false, true, 6>(map, wmap, w2map, p, n_tiles, stream);
+        return launch_staged<DT, false, true, 4>(map, wmap, w2map, p, n_tiles, stream);
+    } else {
+        return gate ? launch_staged<DT, true, false, 3>(map, wmap, w2map, p, n_tiles, stream) : launch_staged<DT, false, false, 4>(map, wmap, w2map, p, n_tiles, stream);
+    }
 }
 
 // Adds the shares of the tiles tile0 .. tile0 + gridDim.x - 1 of a gate / up product in a fixed order and writes silu(gate) * up as f16 (the epilogue of
@@ -566,17 +602,19 @@ cudaError_t dequant_rows_dt(int dt, const void * W, void * out, int64_t rows, in
 
 static_assert(sizeof(TensorMap) == sizeof(CUtensorMap) && alignof(TensorMap) >= alignof(CUtensorMap), "TensorMap must hold a CUtensorMap");
 
-cudaError_t make_activation_map(TensorMap * out, const void * base, int64_t rows, int64_t cols) {
+static cudaError_t make_tile_map(TensorMap * out, const void * base, int64_t rows, int64_t cols, int box_rows) {
     EncodeTiledFn fn = encode_tiled();
     if (!fn) return cudaErrorNotSupported;
     const cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
     const cuuint64_t strides[1] = {cuuint64_t(cols) * 2};
-    const cuuint32_t box[2] = {cuuint32_t(kStepK), 128u};
+    const cuuint32_t box[2] = {cuuint32_t(kStepK), cuuint32_t(box_rows)};
     const cuuint32_t estr[2] = {1u, 1u};
     const CUresult r = fn(reinterpret_cast<CUtensorMap *>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
+
+cudaError_t make_activation_map(TensorMap * out, const void * base, int64_t rows, int64_t cols) { return make_tile_map(out, base, rows, cols, kTokenBox); }
 
 cudaError_t make_rows_map(TensorMap * out, const void * base, int64_t rows, int64_t row_bytes, int box_bytes, int box_rows) {
     EncodeTiledFn fn = encode_tiled();
@@ -597,29 +635,81 @@ static int pre_from_tokens() {
     return v;
 }
 
-static int k_splits_of_rows16(int M, int64_t N, int64_t K);
-
-int gemm_tc_k_splits(int dt, int M, int64_t N, int64_t K, bool gate, size_t w16_bytes) {
-    const bool wide = (dt == kQ4_0 || dt == kQ4_K) && K % 256 == 0;
-    const bool pre = w16_bytes >= size_t(N) * size_t(K) * 2 * (gate ? 2 : 1) && M >= pre_from_tokens() && dt != kF16 && !(wide && gate);
-    if (gate || !pre) return 1;
-    return k_splits_of_rows16(M, N, K);
+// How a product on f16 rows is cut: tokens per block and shares of the reduction. A model of the time in SM cycles, fitted to one-kernel timings: a block's k step
+// costs what its tensor-core instructions and its copies need (kStepCycles), a block its set-up and epilogue besides, and blocks run in waves of one per SM;
+// a split adds its sums' way through L2 and the kernel that adds them. Large products come out as 256-token tiles (the fewest bytes per flop); a product that
+// leaves SMs idle that way takes smaller tiles, or deals its reduction, until they are busy.
+constexpr int kMaxSplits = 32;
+static int64_t wave_cost(int64_t blocks, int64_t block_cycles) { return (blocks + sm_count() - 1) / sm_count() * block_cycles; }
+static int64_t step_cycles(int T, bool gate) { return gate ? (T == 64 ? 700 : T == 128 ? 800 : 1100) : (T == 64 ? 560 : T == 128 ? 610 : 840); }
+static int64_t fixed_cycles(int T, bool gate) { return gate ? (T == 64 ? 8000 : T == 128 ? 12500 : 24000) : (T == 64 ? 5500 : T == 128 ? 6300 : 8000); }
+constexpr int64_t kPairStep = 1450, kPairFixed = 14000;      // a block of 256 weight rows x 256 tokens
+// One matrix, 256 tokens per block: the first token tiles run as blocks of 256 weight rows (two accumulators that share the token tile, which cuts what a block
+// pulls out of L2 per flop by a third), the rest as plain tiles, whichever mix takes the least time; the number of the former comes back.
+static int pair_token_tiles(int M, int64_t N, int64_t K, int64_t * cost) {
+    static const int pair_mode = [] { const char * e = getenv("DOOMS_GEMM_PAIR"); return e ? atoi(e) : -1; }();      // 0: never, 1: always, -1: by the estimate
+    const int token_tiles = (M + 255) / 256;
+    const int64_t single = (N + kRowsW - 1) / kRowsW, pair = (N + 2 * kRowsW - 1) / (2 * kRowsW), ksteps = K / kStepK;
+    int best = 0;
+    *cost = -1;
+    for (int tm = pair_mode > 0 && N > kRowsW ? token_tiles : 0; tm <= (pair_mode == 0 || N <= kRowsW ? 0 : token_tiles); tm++) {
+        const int64_t c = wave_cost(pair * tm, kPairFixed + kPairStep * ksteps) + wave_cost(single * (token_tiles - tm), fixed_cycles(256, false) + ksteps * step_cycles(256, false));
+        if (*cost < 0 || c < *cost) { *cost = c; best = tm; }
+    }
+    return best;
 }
-int gemm_tc_rows16_k_splits(int M, int64_t N, int64_t K) { return k_splits_of_rows16(M, N, K); }
-
-static int k_splits_of_rows16(int M, int64_t N, int64_t K) {
+static int64_t cut_cost(int T, int splits, int M, int64_t N, int64_t K, bool gate) {
+    const int64_t tiles = (N + kRowsW - 1) / kRowsW * ((M + T - 1) / T), ksteps = K / kStepK, per = (ksteps + splits - 1) / splits;
+    int64_t cost = wave_cost(tiles * splits, fixed_cycles(T, gate) + per * step_cycles(T, gate));
+    if (T == 256 && splits == 1 && !gate) (void)pair_token_tiles(M, N, K, &cost);
+    return splits == 1 ? cost : cost + 1000 + int64_t(splits) * M * N * 4 / 1500;
+}
+static bool tile_fits(int T, int M) { return T == 64 || M > T / 2; }
+static int tokens_per_block(int M, int64_t N, int64_t K, bool gate, int splits) {
+    static const int fixed = [] { const char * e = getenv("DOOMS_GEMM_TOKENS"); return e ? atoi(e) : 0; }();
+    if (fixed == 64 || fixed == 128 || fixed == 256) return fixed;
+    int best = 64;
+    for (int T : {128, 256}) if (tile_fits(T, M) && cut_cost(T, splits, M, N, K, gate) <= cut_cost(best, splits, M, N, K, gate)) best = T;
+    return best;
+}
+static int k_splits_of_rows16(int M, int64_t N, int64_t K, int most) {
     static const bool off = [] { const char * e = getenv("DOOMS_GEMM_SPLIT_K"); return e && *e == '0'; }();
     if (off || K % kStepK != 0) return 1;
-    const int T = M > 128 ? 256 : 128;
-    const int64_t tiles = (N + kRowsW - 1) / kRowsW * ((M + T - 1) / T);
     const int ksteps = int(K / kStepK);
-    // worth it when the tiles leave most SMs idle and every share still has a few k steps; shares of equal size, none empty
-    int want = int(std::min<int64_t>(sm_count() / std::max<int64_t>(tiles, 1), ksteps / 4));
-    if (tiles * 2 > sm_count() || want < 2) return 1;
-    want = std::min(want, 32);
-    const int per = (ksteps + want - 1) / want;
-    return (ksteps + per - 1) / per;
+    int best = 1;
+    int64_t best_cost = cut_cost(tokens_per_block(M, N, K, false, 1), 1, M, N, K, false);
+    for (int s = 2; s <= std::min({most, kMaxSplits, ksteps / 4}); s++) {
+        const int per = (ksteps + s - 1) / s;
+        if ((ksteps + per - 1) / per != s) continue;      // shares of equal size, none empty
+        const int64_t cost = cut_cost(tokens_per_block(M, N, K, false, s), s, M, N, K, false);
+        if (cost < best_cost) { best_cost = cost; best = s; }
+    }
+    return best;
 }
+
+static bool wide_rows(int dt, int64_t K, const void * W) { return (dt == kQ4_0 || dt == kQ4_K) && K % 256 == 0 && (reinterpret_cast<uintptr_t>(W) & 15u) == 0; }
+// Whether a product runs on f16 rows: f16 weights always (they are such rows); others from pre_from_tokens() tokens on (see launch_gemm_tc), and at any number of
+// tokens when the format has no wide producers: one element after another in every tile, they pay a memory latency per k step (17 us for the 14 steps of an
+// 896-wide product, 37 us for 76), the pass that writes the rows 3 to 6 us.
+static bool on_rows16(int dt, const void * W, int M, int64_t N, int64_t K, bool gate, size_t w16_bytes) {
+    if (dt == kF16) return (reinterpret_cast<uintptr_t>(W) & 15u) == 0;
+    const bool wide = wide_rows(dt, K, W);
+    return w16_bytes >= size_t(N) * size_t(K) * 2 * (gate ? 2 : 1) && (wide ? M >= pre_from_tokens() && !gate : true);
+}
+
+int gemm_tc_k_splits(int dt, const void * W, int M, int64_t N, int64_t K, size_t w16_bytes, int most) {
+    if (on_rows16(dt, W, M, N, K, false, w16_bytes)) return k_splits_of_rows16(M, N, K, most);
+    if (!wide_rows(dt, K, W)) return 1;
+    // The wide producers: a block takes as long as its k steps (0.45 us each: the groups' loads are a chain of latencies), so a product of few row tiles is dealt over
+    // the idle SMs in shares of whole 256-element groups.
+    const int64_t tiles = (N + kRowsW - 1) / kRowsW * ((M + 255) / 256);
+    const int groups = int(K / 256);
+    const int s = std::min({int(sm_count() / tiles), groups / 4, most, kMaxSplits});
+    if (s < 2) return 1;
+    const int per = (groups + s - 1) / s;
+    return (groups + per - 1) / per;
+}
+int gemm_tc_rows16_k_splits(int M, int64_t N, int64_t K, int most) { return k_splits_of_rows16(M, N, K, most); }
 
 bool gemm_tc_supported(int dt, const void * W, int64_t N, int64_t K) {
     (void)W;
@@ -632,33 +722,22 @@ static cudaError_t launch_rows16(GemmTcParams p, const CUtensorMap & xmap, const
                                  int64_t split_stride, cudaStream_t stream) {
     const bool gate = w2_16 != nullptr;
     TensorMap wmap, w2map;
-    cudaError_t e = make_activation_map(&wmap, w16, N, K);
-    if (e == cudaSuccess) e = make_activation_map(&w2map, gate ? w2_16 : w16, N, K);
+    cudaError_t e = make_tile_map(&wmap, w16, N, K, kRowsW);
+    if (e == cudaSuccess) e = make_tile_map(&w2map, gate ? w2_16 : w16, N, K, kRowsW);
     if (e != cudaSuccess) return e;
     p.wide = 0;
+    p.T = tokens_per_block(M, N, K, gate, k_splits);
     if (k_splits > 1) {
         const int ksteps = int(K / kStepK);
         p.ks_per = (ksteps + k_splits - 1) / k_splits;
         p.split_stride = split_stride;
     }
-    // One matrix: a block may take 256 weight rows (two accumulators that share the token tile), which cuts what a block pulls out of L2 per flop by
-    // a third. A block of 256 rows is taken to cost 1.5 plain tiles; the first `pair_tm` token tiles run as such blocks and the rest as plain tiles,
-    // whichever split needs the least time in waves of one block per SM (the 8B qkv product, 48 x 8 plain tiles: six token tiles as 144 blocks of 256
-    // rows, two as 96 plain tiles, 2.5 units of time against 3 either way alone).
     const CUtensorMap & wm = *reinterpret_cast<const CUtensorMap *>(&wmap), & w2m = *reinterpret_cast<const CUtensorMap *>(&w2map);
-    if (gate || k_splits > 1 || N <= kRowsW) return launch_dt<kF16, true>(xmap, wm, w2m, p, gate, stream);
-    static const int pair_mode = [] { const char * e = getenv("DOOMS_GEMM_PAIR"); return e ? atoi(e) : -1; }();      // 0: never, 1: always, -1: by the estimate
-    const int token_tiles = (M + p.T - 1) / p.T, sms = sm_count();
+    if (gate || k_splits > 1 || N <= kRowsW || p.T != 256) return launch_dt<kF16, true>(xmap, wm, w2m, p, gate, stream);
+    const int token_tiles = (M + p.T - 1) / p.T;
     const int tiles_single = int((N + kRowsW - 1) / kRowsW), tiles_pair = int((N + 2 * kRowsW - 1) / (2 * kRowsW));
-    int pair_tm = 0;
-    if (pair_mode > 0) pair_tm = token_tiles;
-    if (pair_mode < 0) {
-        int64_t best = -1;
-        for (int tm = 0; tm <= token_tiles; tm++) {
-            const int64_t cost = int64_t((tiles_pair * tm + sms - 1) / sms) * 3 + int64_t((tiles_single * (token_tiles - tm) + sms - 1) / sms) * 2;
-            if (best < 0 || cost < best) { best = cost; pair_tm = tm; }
-        }
-    }
+    int64_t cost = 0;
+    const int pair_tm = pair_token_tiles(M, N, K, &cost);
     cudaError_t e2 = cudaSuccess;
     if (pair_tm > 0) {
         GemmTcParams q = p;
@@ -680,7 +759,7 @@ static cudaError_t launch_rows16(GemmTcParams p, const CUtensorMap & xmap, const
 cudaError_t launch_gemm_tc_rows16(const void * W16, const void * W2_16, const TensorMap * xmap, float * Y, void * Y16, const float * bias, int M, int64_t N, int64_t K,
                                   int64_t y_stride, int64_t y16_stride, uint32_t flags, int32_t * error, cudaStream_t stream, int k_splits, int64_t split_stride) {
     if (!W16 || N < 1 || K < kStepK || K % kStepK != 0 || M < 1 || (reinterpret_cast<uintptr_t>(W16) & 15u) || (reinterpret_cast<uintptr_t>(W2_16) & 15u)) return cudaErrorInvalidValue;
-    if (k_splits > 1 && (k_splits != k_splits_of_rows16(M, N, K) || W2_16 || !Y || Y16 || flags || split_stride < int64_t(M) * y_stride)) return cudaErrorInvalidValue;
+    if (k_splits > 1 && (k_splits > kMaxSplits || W2_16 || !Y || Y16 || flags || split_stride < int64_t(M) * y_stride)) return cudaErrorInvalidValue;
     GemmTcParams p{nullptr, nullptr, Y, static_cast<__half *>(Y16), bias, N, int(K), M, y_stride, y16_stride, flags, M > 128 ? 256 : 128, 0, 0, 0, 0, 0, 0, nullptr, error};
     return launch_rows16(p, *reinterpret_cast<const CUtensorMap *>(xmap), static_cast<const __half *>(W16), static_cast<const __half *>(W2_16), M, N, K, k_splits,
                          split_stride, stream);
@@ -695,28 +774,33 @@ cudaError_t launch_gemm_tc(int dt, const void * W, const void * W2, const Tensor
                            int64_t y_stride, int64_t y16_stride, uint32_t flags, int32_t * error, cudaStream_t stream, void * w16_scratch, size_t w16_bytes, int k_splits,
                            int64_t split_stride) {
     if (!gemm_tc_supported(dt, W, N, K) || M < 1) return cudaErrorInvalidValue;
-    if (k_splits > 1 && (k_splits != gemm_tc_k_splits(dt, M, N, K, W2 != nullptr, w16_scratch ? w16_bytes : 0) || !Y || Y16 || flags || split_stride < int64_t(M) * y_stride)) {
-        return cudaErrorInvalidValue;
-    }
+    if (k_splits > 1 && (k_splits > kMaxSplits || W2 || !Y || Y16 || flags || split_stride < int64_t(M) * y_stride)) return cudaErrorInvalidValue;
     GemmTcParams p{static_cast<const uint8_t *>(W), static_cast<const uint8_t *>(W2), Y, static_cast<__half *>(Y16), bias, N, int(K), M, y_stride, y16_stride,
-                   flags, M > 128 ? 256 : 128, 0, 0, 0, 0, 0, 0, nullptr, error};
-    p.wide = (dt == kQ4_0 || dt == kQ4_K) && K % 256 == 0 && (reinterpret_cast<uintptr_t>(W) & 15u) == 0 && (!W2 || (reinterpret_cast<uintptr_t>(W2) & 15u) == 0) ? 1 : 0;
+                   flags, M > 128 ? 256 : M > 64 ? 128 : 64, 0, 0, 0, 0, 0, 0, nullptr, error};
+    p.wide = wide_rows(dt, K, W) && (!W2 || wide_rows(dt, K, W2)) ? 1 : 0;
     const CUtensorMap & map = *reinterpret_cast<const CUtensorMap *>(xmap);
     const bool gate = W2 != nullptr;
     // Many tokens: dequantize the matrix once to f16 rows and let TMA feed both operands (the reference does the same from 320 tokens on,
     // metal_llama_decoder.mm:31); otherwise every token tile would redo the dequantization in its producer warps.
-    const size_t need = size_t(N) * size_t(K) * 2 * (gate ? 2 : 1);
     // (from 128 tokens: a batched decode step of 256 rows on the 0.5B shape measured 6.4 ms with the weights dequantized by each block's producer warps
     // and 5.5 ms from f16 rows; with few blocks per matrix the producers' loads are a chain of memory latencies)
-    const int pre_from = pre_from_tokens();
     // Measured on the 8B shapes: q4_0 / q4_K gate/up is faster fused (875 against 836 TFLOP/s: no f16 copy to write and read), everything else is faster
     // or much faster from f16 rows (ffn_down 961 against 925; q6_K 754 against 83).
-    if (w16_scratch && need <= w16_bytes && M >= pre_from && dt != kF16 && !(p.wide && gate)) {
+    if (dt == kF16 && on_rows16(dt, W, M, N, K, gate, 0) && (!W2 || (reinterpret_cast<uintptr_t>(W2) & 15u) == 0)) {
+        return launch_rows16(p, map, static_cast<const __half *>(W), static_cast<const __half *>(W2), M, N, K, k_splits, split_stride, stream);
+    }
+    if (dt != kF16 && w16_scratch && on_rows16(dt, W, M, N, K, gate, w16_bytes)) {
         __half * w16 = static_cast<__half *>(w16_scratch);
         cudaError_t e = dequant_rows_dt(dt, W, w16, N, K, stream);
         if (e == cudaSuccess && gate) e = dequant_rows_dt(dt, W2, w16 + size_t(N) * size_t(K), N, K, stream);
         if (e != cudaSuccess) return e;
         return launch_rows16(p, map, w16, gate ? w16 + size_t(N) * size_t(K) : nullptr, M, N, K, k_splits, split_stride, stream);
+    }
+    if (k_splits > 1) {      // (wide producers, see gemm_tc_k_splits)
+        if (!p.wide) return cudaErrorInvalidValue;
+        const int groups = int(K / 256);
+        p.ks_per = (groups + k_splits - 1) / k_splits * 4;
+        p.split_stride = split_stride;
     }
     switch (dt) {
         case kF16: return launch_dt<kF16, false>(map, map, map, p, gate, stream);

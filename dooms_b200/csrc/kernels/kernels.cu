@@ -78,11 +78,12 @@ __global__ void k_embed(const uint8_t * table, const int32_t * ids, const int32_
 // Many rows (a prefill chunk, a batched step) take blocks of 256 threads with up to 16 elements each: eight blocks share an SM and cover each other's
 // round trips, where 1024-thread blocks ran in waves of two per SM (22 us for 2048 rows of 4096 floats; the bytes alone are 8 us).
 template <int kNormThreads, int kNormMaxPerThread>
-__global__ void __launch_bounds__(kNormThreads) k_rms_norm(const float * x, const float * gamma, float * out, __half * out16, uint8_t * xq, int E, float eps) {
+__global__ void __launch_bounds__(kNormThreads) k_rms_norm(float * x, const float * gamma, float * out, __half * out16, uint8_t * xq, int E, float eps,
+                                                            const float * shares, int n_shares, int64_t share_stride) {
     pdl_trigger();
     pdl_wait();
     __shared__ float red[kNormThreads / 32];
-    const float * xr = x + int64_t(blockIdx.x) * E;
+    float * xr = x + int64_t(blockIdx.x) * E;
     const int64_t obase = int64_t(blockIdx.x) * E;
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
     float ss = 0.f;
@@ -93,6 +94,21 @@ __global__ void __launch_bounds__(kNormThreads) k_rms_norm(const float * x, cons
             const int i = k * kNormThreads + threadIdx.x;
             v[k] = i < E ? xr[i] : 0.f;
             g[k] = i < E ? gamma[i] : 0.f;
+        }
+        if (n_shares > 0) {
+            #pragma unroll 4
+            for (int z = 0; z < n_shares; z++) {
+                #pragma unroll
+                for (int k = 0; k < kNormMaxPerThread; k++) {
+                    const int i = k * kNormThreads + threadIdx.x;
+                    if (i < E) v[k] += __ldcg(shares + int64_t(z) * share_stride + obase + i);
+                }
+            }
+            #pragma unroll
+            for (int k = 0; k < kNormMaxPerThread; k++) {
+                const int i = k * kNormThreads + threadIdx.x;
+                if (i < E) xr[i] = v[k];
+            }
         }
         #pragma unroll
         for (int k = 0; k < kNormMaxPerThread; k++) ss += v[k] * v[k];
@@ -116,7 +132,12 @@ __global__ void __launch_bounds__(kNormThreads) k_rms_norm(const float * x, cons
         }
         return;
     }
-    for (int i = threadIdx.x; i < E; i += kNormThreads) { const float t = xr[i]; ss += t * t; }
+    for (int i = threadIdx.x; i < E; i += kNormThreads) {
+        float t = xr[i];
+        for (int z = 0; z < n_shares; z++) t += __ldcg(shares + int64_t(z) * share_stride + obase + i);
+        if (n_shares > 0) xr[i] = t;      // (read again below by the thread that wrote it)
+        ss += t * t;
+    }
     ss = warp_sum(ss);
     if (lane == 0) red[warp] = ss;
     __syncthreads();
@@ -522,12 +543,20 @@ cudaError_t launch_embed(int dt, const void * table, const int32_t * ids, const 
     return ok ? e : cudaErrorInvalidValue;
 }
 
-cudaError_t launch_rms_norm(const float * x, const float * gamma, float * out, void * out16, void * xq, int rows, int E, float eps, cudaStream_t stream) {
-    if (xq && (rows != 1 || E % 32 != 0)) return cudaErrorInvalidValue;
-    if (rows >= 64 && E <= 256 * 16) {
-        return launch_pdl(k_rms_norm<256, 16>, dim3(rows), dim3(256), 0, stream, x, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps);
+cudaError_t launch_rms_norm(const float * x, const float * gamma, float * out, void * out16, void * xq, int rows, int E, float eps, cudaStream_t stream,
+                            const float * shares, int n_shares, int64_t share_stride) {
+    if ((xq && (rows != 1 || E % 32 != 0)) || (n_shares > 0 && !shares)) return cudaErrorInvalidValue;
+    float * const xw = const_cast<float *>(x);
+    if (rows >= 64 && E <= 256 * 4) {      // (few registers: the shares of four products are loaded together)
+        return launch_pdl(k_rms_norm<256, 4>, dim3(rows), dim3(256), 0, stream, xw, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps,
+                          shares, n_shares, share_stride);
     }
-    return launch_pdl(k_rms_norm<1024, 8>, dim3(rows), dim3(1024), 0, stream, x, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps);
+    if (rows >= 64 && E <= 256 * 16) {
+        return launch_pdl(k_rms_norm<256, 16>, dim3(rows), dim3(256), 0, stream, xw, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps,
+                          shares, n_shares, share_stride);
+    }
+    return launch_pdl(k_rms_norm<1024, 8>, dim3(rows), dim3(1024), 0, stream, xw, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps,
+                          shares, n_shares, share_stride);
 }
 
 cudaError_t launch_matvec(int dt, const void * W, const float * x, float * y, const float * bias, int64_t rows, int64_t cols, uint32_t flags, cudaStream_t stream) {

@@ -40,7 +40,10 @@ cudaError_t launch_embed(int dt, const void * table, const int32_t * ids, const 
 
 // out[r][:] = x[r][:] * rsqrt(mean(x[r]^2) + eps) * gamma (norm_vec, llama_kernels.h:1272-1286). out16 (optional) also receives the rows as f16; xq
 // (optional, one row, E a multiple of 32) the row split for the staged q4_0 GEMV.
-cudaError_t launch_rms_norm(const float * x, const float * gamma, float * out, void * out16, void * xq, int rows, int E, float eps, cudaStream_t stream);
+// n_shares > 0: x[r] += the sum of the n_shares row blocks shares[z][r] (share_stride floats apart, added in that order) first, left in x: the residual add of a
+// product that was dealt over several blocks per tile (launch_gemm_tc with k_splits), without a pass of its own (x is written then, and only then).
+cudaError_t launch_rms_norm(const float * x, const float * gamma, float * out, void * out16, void * xq, int rows, int E, float eps, cudaStream_t stream,
+                            const float * shares = nullptr, int n_shares = 0, int64_t share_stride = 0);
 
 // y[r] (+)= W[r] . x (+ bias[r]) (matvec1q<Q>, llama_kernels.h:1197-1230).
 cudaError_t launch_matvec(int dt, const void * W, const float * x, float * y, const float * bias, int64_t rows, int64_t cols, uint32_t flags, cudaStream_t stream);
@@ -245,19 +248,20 @@ cudaError_t make_rows_map(TensorMap * out, const void * base, int64_t rows, int6
 bool gemm_tc_supported(int dt, const void * W, int64_t N, int64_t K);
 // Y[m][n] (+)= X[m] . W[n] (+ bias[n]) for M tokens; X is the f16 buffer behind xmap. With W2: silu(X . W[n]) * (X . W2[n]). Y (f32) and / or Y16 (f16)
 // receive the result. *error is set to 2 if a pipeline wait ran out.
-// w16_scratch (optional, w16_bytes): room for the matrix (both, for gate/up) as f16 rows; with it and 512 or more tokens the weights are dequantized once
-// per call and both operands arrive by TMA.
+// w16_scratch (optional, w16_bytes): room for the matrix (both, for gate/up) as f16 rows; with it the weights are dequantized once per call and both operands
+// arrive by TMA where that is faster (f16 weights need no copy and always arrive that way).
 cudaError_t launch_gemm_tc(int dt, const void * W, const void * W2, const TensorMap * xmap, float * Y, void * Y16, const float * bias, int M, int64_t N, int64_t K,
                            int64_t y_stride, int64_t y16_stride, uint32_t flags, int32_t * error, cudaStream_t stream,
                            void * w16_scratch = nullptr, size_t w16_bytes = 0, int k_splits = 1, int64_t split_stride = 0);
 // A product whose tiles would leave most SMs idle (few weight rows against one token tile: a batched decode step) can deal its reduction dimension over
 // k_splits blocks per tile: gemm_tc_k_splits says how many (1: do not split), launch_gemm_tc with that k_splits then writes the shares' sums to
 // Y + z * split_stride (flags 0, no f16 output), and launch_add_shares adds them onto x in a fixed order, so the result does not depend on timing.
-int gemm_tc_k_splits(int dt, int M, int64_t N, int64_t K, bool gate, size_t w16_bytes);
+// most: how many shares the caller has room for.
+int gemm_tc_k_splits(int dt, const void * W, int M, int64_t N, int64_t K, size_t w16_bytes, int most);
 // The same product against weights that already lie in device memory as f16 rows [N][K] (W2_16: the second matrix of a gate / up pair): a decoder that
 // runs batched steps keeps such a copy of its matrices, made once with launch_dequant_rows16, instead of dequantizing them in every step.
 cudaError_t launch_dequant_rows16(int dt, const void * W, void * out, int64_t rows, int64_t cols, cudaStream_t stream);
-int gemm_tc_rows16_k_splits(int M, int64_t N, int64_t K);
+int gemm_tc_rows16_k_splits(int M, int64_t N, int64_t K, int most);
 cudaError_t launch_gemm_tc_rows16(const void * W16, const void * W2_16, const TensorMap * xmap, float * Y, void * Y16, const float * bias, int M, int64_t N, int64_t K,
                                   int64_t y_stride, int64_t y16_stride, uint32_t flags, int32_t * error, cudaStream_t stream, int k_splits = 1, int64_t split_stride = 0);
 cudaError_t launch_add_shares(float * x, const float * shares, int k_splits, int64_t n, int64_t split_stride, cudaStream_t stream);
