@@ -51,7 +51,23 @@ cudaError_t launch_staged(const AttnDecodeParams & p, cudaStream_t stream) {
     constexpr size_t smem = attention_decode_smem_bytes<D, GP, STAGES>();
     static std::atomic<uint64_t> configured{0};
     if (const cudaError_t e = allow_dynamic_smem(k_attention_decode<D, GP, STAGES>, int(smem), configured); e != cudaSuccess) return e;
-    return launch_pdl(k_attention_decode<D, GP, STAGES>, dim3(p.s.n_head_kv, p.splits, p.b_slot ? unsigned(p.b_rows) : 1u), dim3(kThreads), smem, stream, p);
+    if (!p.cluster) return launch_pdl(k_attention_decode<D, GP, STAGES>, dim3(p.s.n_head_kv, p.splits, p.b_slot ? unsigned(p.b_rows) : 1u), dim3(kThreads), smem, stream, p);
+    // clusters of kCluster consecutive ranges; the grid is rounded up to whole clusters, blocks past the last range leave at once
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.s.n_head_kv, (p.splits + kCluster - 1) / kCluster * kCluster, 1);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = kCluster;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, k_attention_decode<D, GP, STAGES>, p);
 }
 
 template <int D, int GP>
@@ -91,6 +107,8 @@ cudaError_t launch_attention_gqa(const float * qkv, void * kc, void * vc, float 
     AttnDecodeParams p{qkv, static_cast<__half *>(kc), static_cast<__half *>(vc), part, st, inv_freq, n_keys_fixed, splits, s, counters, out,
                        static_cast<uint8_t *>(xq), static_cast<const float2 *>(rope_cs), nullptr, nullptr, 0, 0, 0, nullptr, 0};
     p.cache_ready = cache_keys;
+    static const bool clusters = [] { const char * e = getenv("DOOMS_ATTN_CLUSTER"); return !(e && *e == '0'); }();
+    p.cluster = clusters && cache_keys && counters && splits > 1 ? 1 : 0;
     return s.head_dim == 64 ? launch_group<64>(p, s.n_head / s.n_head_kv, stream) : launch_group<128>(p, s.n_head / s.n_head_kv, stream);
 }
 

@@ -19,6 +19,8 @@ constexpr int kThreads = 256;
 constexpr int kTileKeys = 64;
 constexpr int kStagesFull = 4;      // two pairs of tiles: the block's 8 warps work on one pair while the next is on its way
 
+constexpr int kCluster = 8;     // ranges whose blocks can read one another's shared memory
+
 struct AttnDecodeParams {
     const float * qkv;        // the new token's row: query heads, then key heads, then value heads
     __half * kc;
@@ -45,10 +47,22 @@ struct AttnDecodeParams {
     // Single-row decode inside a step whose position was final before this kernel could start (launch_attention_gqa): the cached keys and values of earlier
     // positions do not depend on the projection in front of this kernel, so a block asks for its range before it waits for that projection. The row of the
     // new position is whatever the cache held; it is overwritten in shared memory once the projection is done, as it always was.
+    int cluster;              // the blocks of kCluster consecutive ranges of a key/value head form a thread-block cluster
     int cache_ready;          // the positions the caches have room for (0: not so)
 };
 
 __device__ __forceinline__ void cp16(uint32_t dst, const void * src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cluster_barrier() {      // all threads of the cluster's blocks that have not left
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {      // the float at shared-memory address addr of block `rank` of the cluster
+    uint32_t at;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t & r0, uint32_t & r1, uint32_t & r2, uint32_t & r3) {
@@ -100,7 +114,7 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
     constexpr int OUT_IT = (GP * D / 2 + kThreads - 1) / kThreads;   // (head, dim pair) outputs per thread
     constexpr int MERGE_IT = (GP * D + kThreads - 1) / kThreads;     // single outputs per thread in the merge
     constexpr int RS = 2 + D;                                          // floats per head in the warps' results
-    static_assert(GP <= 8 && size_t(8) * 8 * RS * 4 <= size_t(kStages) * STAGE, "the warps' results are laid over the stages");
+    static_assert(GP <= 8 && size_t(9) * 8 * RS * 4 <= size_t(kStages) * STAGE, "the warps' results and the block's are laid over the stages");
     __half * Qh = reinterpret_cast<__half *>(smem);                    // [8 heads: values][LD], then [8 heads: rounding errors][LD]
     uint8_t * stages = smem + 16 * LD * 2;
     const uint32_t stages_u = smem_u32(stages);
@@ -364,6 +378,41 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
         }
     }
     cp_wait<0>();
+    if (p.cluster && used <= kCluster) {
+        // All ranges that hold keys belong to one cluster (its first `used` blocks; the others have left): the results stay in shared memory, and each block merges
+        // its share of the heads' 32-element blocks out of everybody's. Through device memory the same merge is a fence, an atomic, a barrier and two round trips
+        // to L2 on one block per key/value head (0.5B shape at 580 keys, five ranges: 7.5 us a launch against 3.6 at one range).
+        float * mine = res + 64 * RS;                     // [head][2 + D], behind the warps' results
+        #pragma unroll
+        for (int it = 0; it < OUT_IT; it++) {
+            const int idx = tid + it * kThreads;
+            if (idx < GP * D / 2) *reinterpret_cast<float2 *>(mine + (idx / (D / 2)) * RS + 2 + 2 * (idx % (D / 2))) = make_float2(acc[it][0], acc[it][1]);
+        }
+        if (warp < GP && lane == 0) { mine[warp * RS] = m_run; mine[warp * RS + 1] = l_run; }
+        cluster_barrier();
+        for (int b = split + used * warp; b < G * D / 32; b += used * (kThreads / 32)) {
+            const int hq = b * 32 / D, d = b * 32 % D + lane;
+            const uint32_t at = smem_u32(mine + hq * RS);
+            float m[kCluster], l[kCluster], v[kCluster];
+            #pragma unroll
+            for (int r = 0; r < kCluster; r++) {
+                if (r < used) { m[r] = ld_cluster(at, r); l[r] = ld_cluster(at + 4, r); v[r] = ld_cluster(at + 4 * (2 + d), r); }
+                else { m[r] = -CUDART_INF_F; l[r] = v[r] = 0.f; }
+            }
+            float mx = -CUDART_INF_F, total = 0.f, sum = 0.f;
+            #pragma unroll
+            for (int r = 0; r < kCluster; r++) if (l[r] > 0.f) mx = fmaxf(mx, m[r]);
+            #pragma unroll
+            for (int r = 0; r < kCluster; r++) {
+                const float w = l[r] > 0.f ? expf(m[r] - mx) : 0.f;
+                total += l[r] * w;
+                sum += v[r] * w;
+            }
+            finish(hq, d, sum / total);
+        }
+        cluster_barrier();                                // nobody leaves while its results are being read
+        return;
+    }
     // partial results
     #pragma unroll
     for (int it = 0; it < OUT_IT; it++) {
