@@ -624,7 +624,8 @@ struct CudaLlamaDecoder::Impl {
                 const bool split_attn = takes_split(L.attn_output) && cfg.head_dim % 32 == 0 && (gqa || splits > 1) && attn_width == q_width;
                 if (gqa) {
                     run("attention", [&] {
-                        return cuda::launch_attention_gqa(qkv, kcl, vcl, part, state, inv_freq, 0, gqa_splits, as, attn_counters, attn + attn_pad, split_attn ? xq : nullptr, stream, rope_cs, cfg.n_ctx);
+                        return cuda::launch_attention_gqa(qkv, kcl, vcl, part, state, inv_freq, 0, gqa_splits, as, attn_counters, attn + attn_pad, split_attn ? xq : nullptr, stream, rope_cs, cfg.n_ctx,
+                                                          short_qkv(L));
                     });
                 } else {
                     run("rope_store", [&] { return cuda::launch_rope_store(qkv, kcl, vcl, state, inv_freq, 1, as, stream); });

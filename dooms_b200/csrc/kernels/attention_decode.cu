@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(kThreads) k_attention_decode(const AttnDecodeP
     attention_decode_body<D, GP, true, STAGES>(pp, int(blockIdx.x), int(blockIdx.y), int(blockIdx.z), smem);
 }
 
-// Heads of 128 on a context of which a range holds one pair of tiles at most: two stages are all such a block uses, and 74 KB instead of 143 leave it room beside
-// the projection in front, so that its fetches are early (the 8B shape at 60 keys: 10.3 us to 6.0). Longer ranges want the second pair on its way (the 32B shape
+// Heads of 128 on a context of which a range holds two pairs of tiles at most: two stages, and 74 KB instead of 143, leave a block room beside the projection in
+// front, so that its fetches are early (the 8B shape at 60 keys: 10.3 us to 6.0). Longer ranges want the second pair on its way (the 32B shape
 // at 8200 keys, ranges of four pairs: 24.1 us with four stages, 28.4 with two, also with twice as many blocks).
 template <int D, int GP, int STAGES>
 cudaError_t launch_staged(const AttnDecodeParams & p, cudaStream_t stream) {
@@ -73,7 +73,7 @@ cudaError_t launch_staged(const AttnDecodeParams & p, cudaStream_t stream) {
 template <int D, int GP>
 cudaError_t launch_one(const AttnDecodeParams & p, cudaStream_t stream) {
     if constexpr (D > 64) {
-        if (p.cache_ready && p.cache_ready <= p.splits * 2 * kTileKeys) return launch_staged<D, GP, 2>(p, stream);
+        if (p.cache_ready && p.cache_ready <= p.splits * 4 * kTileKeys) return launch_staged<D, GP, 2>(p, stream);
     }
     return launch_staged<D, GP, kStagesFull>(p, stream);
 }
@@ -102,13 +102,13 @@ int attention_gqa_splits(int n_head_kv, int n_ctx) {
 }
 
 cudaError_t launch_attention_gqa(const float * qkv, void * kc, void * vc, float * part, const DevState * st, const double * inv_freq, int n_keys_fixed,
-                                 int splits, const AttnShape & s, int * counters, float * out, void * xq, cudaStream_t stream, const void * rope_cs, int cache_keys) {
+                                 int splits, const AttnShape & s, int * counters, float * out, void * xq, cudaStream_t stream, const void * rope_cs, int cache_keys, bool clusters) {
     if (!attention_gqa_supported(s) || (!inv_freq && n_keys_fixed < 1) || (counters && !out) || (xq && !counters) || cache_keys < 0 || (cache_keys && (!st || !inv_freq))) return cudaErrorInvalidValue;
     AttnDecodeParams p{qkv, static_cast<__half *>(kc), static_cast<__half *>(vc), part, st, inv_freq, n_keys_fixed, splits, s, counters, out,
                        static_cast<uint8_t *>(xq), static_cast<const float2 *>(rope_cs), nullptr, nullptr, 0, 0, 0, nullptr, 0};
     p.cache_ready = cache_keys;
-    static const bool clusters = [] { const char * e = getenv("DOOMS_ATTN_CLUSTER"); return !(e && *e == '0'); }();
-    p.cluster = clusters && cache_keys && counters && splits > 1 ? 1 : 0;
+    static const bool off = [] { const char * e = getenv("DOOMS_ATTN_CLUSTER"); return e && *e == '0'; }();
+    p.cluster = clusters && !off && counters && splits > 1 ? 1 : 0;
     return s.head_dim == 64 ? launch_group<64>(p, s.n_head / s.n_head_kv, stream) : launch_group<128>(p, s.n_head / s.n_head_kv, stream);
 }
 
