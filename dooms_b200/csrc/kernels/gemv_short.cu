@@ -37,7 +37,7 @@ constexpr int kTileRows = 16;
 constexpr int kHeld = 8;                       // input blocks a warp keeps in registers while it normalizes: rows of up to 2048 make one pass
 constexpr int64_t kOwnNorm = int64_t(kHeld) * kWarps * 32;
 constexpr int kMaxRows = 64;                   // rows per block
-constexpr size_t kSmemLimit = 96 * 1024;       // two blocks per SM always fit, whatever kernel they belong to
+constexpr size_t kSmemLimit = 92 * 1024;       // two blocks per SM always fit, whatever kernel they belong to
 
 struct Input {
     const uint8_t * xq;      // the split input, or
@@ -80,7 +80,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 template <int WARPS>
 __device__ __forceinline__ void load_gains(const Input & in, float (&gm)[kHeld]) {
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nb = in.cols / 32;
-    if (in.gamma && nb <= kHeld * WARPS) {
+    if (in.gamma) {
         #pragma unroll
         for (int j = 0; j < kHeld; j++) {
             const int blk = warp + j * WARPS;
@@ -103,57 +103,43 @@ __device__ __forceinline__ void prepare_input(const Input & in, float (&gm)[kHel
         cp_async_commit();
         return;
     }
-    const bool one_pass = nb <= kHeld * WARPS;
-    float inv = 1.f, v[kHeld];
-    if (one_pass) {
-        #pragma unroll
-        for (int j = 0; j < kHeld; j++) {
-            const int blk = warp + j * WARPS;
-            v[j] = blk < nb ? __ldcg(in.x + blk * 32 + lane) : 0.f;
-        }
-    }
-    if (in.gamma) {
-        float ss = 0.f;
-        if (one_pass) {
-            #pragma unroll
-            for (int j = 0; j < kHeld; j++) ss += v[j] * v[j];
-        } else {
-            for (int i = tid; i < in.cols; i += THREADS) { const float e = __ldcg(in.x + i); ss += e * e; }
-        }
-        #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) red[warp] = ss;
-        __syncthreads();
-        float total = 0.f;
-        #pragma unroll
-        for (int w = 0; w < WARPS; w++) total += red[w];
-        inv = rsqrtf(total / float(in.cols) + in.eps);
-    }
+    // The norm's factor waits until after the product, W (s u) = s (W u): the row goes into shared memory with its gains alone, and the sums of squares meet the
+    // other warps' at the barrier that the row needs anyway (input_scale).
     auto put = [&](float e, int blk) {
         if constexpr (HALF) reinterpret_cast<float *>(smem)[blk * 32 + lane] = e;
         else split_block(e, lane, blk, nb, smem);
     };
-    if (one_pass) {
-        #pragma unroll
-        for (int j = 0; j < kHeld; j++) {
-            const int blk = warp + j * WARPS;
-            if (blk < nb) put(in.gamma ? v[j] * inv * gm[j] : v[j], blk);
-        }
-        return;
-    }
+    float ss = 0.f;
     for (int blk0 = warp; blk0 < nb; blk0 += WARPS * kHeld) {      // kHeld loads on their way before the first block is used
+        float v[kHeld];
         #pragma unroll
         for (int j = 0; j < kHeld; j++) {
             const int blk = blk0 + j * WARPS;
             v[j] = blk < nb ? __ldcg(in.x + blk * 32 + lane) : 0.f;
-            gm[j] = (in.gamma && blk < nb) ? __ldg(in.gamma + blk * 32 + lane) : 0.f;
+            if (blk0 != warp) gm[j] = (in.gamma && blk < nb) ? __ldg(in.gamma + blk * 32 + lane) : 0.f;
         }
         #pragma unroll
         for (int j = 0; j < kHeld; j++) {
             const int blk = blk0 + j * WARPS;
-            if (blk < nb) put(in.gamma ? v[j] * inv * gm[j] : v[j], blk);
+            ss += v[j] * v[j];
+            if (blk < nb) put(in.gamma ? v[j] * gm[j] : v[j], blk);
         }
     }
+    if (in.gamma) {
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) red[warp] = ss;
+    }
+}
+// After the barrier: what the results are multiplied by. norm_scale: link_scale's, when the producer made the sums.
+template <int WARPS>
+__device__ __forceinline__ float input_scale(const Input & in, const float * red, float norm_scale) {
+    if (in.ss) return norm_scale;
+    if (!in.gamma) return 1.f;
+    float total = 0.f;
+    #pragma unroll
+    for (int w = 0; w < WARPS; w++) total += red[w];
+    return rsqrtf(total / float(in.cols) + in.eps);
 }
 
 // The factor of a norm whose gains the producer of the split applied: its per-block sums, added in a fixed order by one warp.
@@ -179,7 +165,7 @@ __device__ __forceinline__ void fetch_unit(const uint8_t * base, uint32_t dst, i
 // The chunk's pairs of blocks for the lane's rows.
 template <int DT>
 __device__ __forceinline__ void unit_pairs(uint32_t base0, uint32_t base1, uint32_t ba, uint32_t sa, uint32_t t, bool first, int npairs, float & acc0, float & acc1) {
-    #pragma unroll 2
+    #pragma unroll 4      // (a warp's pairs are one chain of loads, MMAs and conversions after another; two at a time: 70.3 instead of 65.0 ms for 512 + 128 tokens of 0.5B)
     for (int pr = 0; pr < npairs; pr++) {
         pair_step_of<DT>(base0, base1, ba, sa, t, first, acc0, acc1);
         base0 += 2 * BlockInfo<DT>::bytes;
@@ -228,7 +214,7 @@ __device__ __forceinline__ void unit_dot(int dt, const uint8_t * smem, uint32_t 
 
 // HALF: f16 weights, the input as f32 in shared memory; otherwise block formats and the input as digits.
 template <bool HALF>
-__global__ void __launch_bounds__(kThreads, 3) k_gemv_short(const __grid_constant__ ShortParams p) {
+__global__ void __launch_bounds__(kThreads, 2) k_gemv_short(const __grid_constant__ ShortParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float red[kWarps];
     __shared__ float norm_scale;
@@ -305,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_gemv_short(const __grid_constan
         float s = 0.f;
         #pragma unroll
         for (int w = 0; w < kWarps; w++) s += src[w * kTileRows];
-        const float scale = p.in.ss ? norm_scale : 1.f;
+        const float scale = input_scale<kWarps>(p.in, red, norm_scale);
         s *= scale;
         if (nmat == 2) {
             float s2 = 0.f;
@@ -374,7 +360,7 @@ __global__ void __launch_bounds__(kTallWarps * 32, 1) k_gemv_tall(const __grid_c
     }
     cp_async_wait<0>();
     __syncthreads();
-    const float scale = p.in.ss ? norm_scale : 1.f;
+    const float scale = input_scale<kTallWarps>(p.in, red, norm_scale);
     const int g = lane >> 2, t = lane & 3;
     for (; tile < tile_end; tile += kTallWarps) {
         const int64_t row0 = int64_t(tile) * kTileRows;
@@ -451,9 +437,11 @@ Plan plan_for(int dt, int64_t rows, int64_t all_rows, int64_t cols, int nmat, bo
     const int sms = sm_count();
     int rpb = int((all_rows + sms - 1) / sms);
     if (rpb > 8) rpb = std::min(kMaxRows, (rpb + kTileRows - 1) / kTileRows * kTileRows);
+    // A gate / up pair may take up to three smaller blocks per SM. A plain projection that does not fit one per SM is left to the ring kernels: the 8B shape's qkv and
+    // attn_output, two and three blocks per SM here, made no difference after a prompt of 2048 tokens and cost 0.8 of 84.0 ms at a short one.
     for (;; rpb /= 2) {
         const Plan pl = plan_rows(dt, rows, cols, nmat, rpb);
-        if (pl.ok || rpb <= 8) return pl;
+        if (pl.ok || rpb <= 8 || nmat == 1) return pl;
     }
 }
 bool fits(const Plan & pl) { return pl.ok && int64_t(pl.blocks) <= int64_t(sm_count()) * std::min<int64_t>(3, int64_t((224 * 1024) / (pl.smem + 1024))); }

@@ -1,0 +1,111 @@
+"""The kernels of small and tall decode projections, the token tiles and shares of the prefill GEMM, and the merge of a step's attention ranges, at the sizes where
+they change over: one row, ragged tiles, the first size past one wave, contexts around a range's and a cluster's end."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from dooms_b200 import CudaLlamaDecoder, synth
+from dooms_b200 import _lib as L
+from helpers import rel_l2, write
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+SHORT_TYPES = [L.F16, L.Q4_0, L.Q5_0, L.Q8_0]
+U = 2.0 ** -24
+
+
+def _matrix(dtype, rows, cols, seed):
+    """(block bytes, the values they stand for in f64), both on the GPU."""
+    from dooms_b200.quantize import quantize
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    w = quantize(dtype, torch.randn(rows, cols, device="cuda", generator=gen) * 0.02)
+    values = torch.empty(rows, cols, device="cuda")
+    L.check(L.lib().dooms_cuda_dequantize(dtype, w.data_ptr(), rows, cols, values.data_ptr(), 0))
+    return w, values.double()
+
+
+def _bound(dtype, values, x):
+    """What f32 sums over blocks (f16: over elements, two to four chains a row) and the input's 27 digits below a block's largest allow, row by row."""
+    cols = values.shape[1]
+    adds = cols / 2 + 32 if dtype == L.F16 else cols / 32 + 32
+    largest = x.abs().view(-1, 32).amax(1).repeat_interleave(32).double()
+    return adds * U * (values.abs() @ x.abs().double()) + 2 * U * (values.abs() @ largest) + 1e-30
+
+
+@pytest.mark.parametrize("dtype", SHORT_TYPES)
+@pytest.mark.parametrize("rows,cols", [(1, 64), (7, 896), (8, 896), (9, 896), (149, 896), (896, 4864), (1153, 896), (18945, 128), (18977, 896)])
+def test_matvec_of_small_and_tall_matrices(dtype, rows, cols):
+    w, values = _matrix(dtype, rows, cols, rows + cols)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(cols, device="cuda", generator=gen)
+    bias = torch.randn(rows, device="cuda", generator=gen)
+    y = torch.full((rows,), 0.5, device="cuda")
+    L.check(L.lib().dooms_cuda_matvec(dtype, w.data_ptr(), x.data_ptr(), y.data_ptr(), bias.data_ptr(), rows, cols, 2 | 4, 0))      # y += W x + bias
+    ref = values @ x.double()
+    err = (y.double() - (ref + bias.double() + 0.5)).abs()
+    assert bool((err <= _bound(dtype, values, x) + 4 * U * (ref.abs() + bias.abs().double() + 1)).all())
+
+
+@pytest.mark.parametrize("dtype", SHORT_TYPES)
+@pytest.mark.parametrize("rows,cols", [(1, 64), (32, 896), (4864, 896), (33, 256)])
+def test_gate_up_of_small_matrices(dtype, rows, cols):
+    wg, vg = _matrix(dtype, rows, cols, 1)
+    wu, vu = _matrix(dtype, rows, cols, 2)
+    x = torch.randn(cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(6)) * 10
+    h = torch.empty(rows, device="cuda")
+    L.check(L.lib().dooms_cuda_gate_up(dtype, wg.data_ptr(), wu.data_ptr(), x.data_ptr(), h.data_ptr(), rows, cols, 0))
+    g, u = vg @ x.double(), vu @ x.double()
+    bg, bu = _bound(dtype, vg, x), _bound(dtype, vu, x)
+    ref = torch.nn.functional.silu(g) * u
+    # silu is 1.1-Lipschitz and at most |g|; exp, divide and the two products round to a few ulp
+    assert bool(((h.double() - ref).abs() <= 1.1 * bg * (u.abs() + bu) + g.abs() * bu + 16 * U * ref.abs() + 1e-30).all())
+
+
+@pytest.mark.parametrize("dtype", SHORT_TYPES)
+@pytest.mark.parametrize("rows", [64, 18977])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_an_input_that_is_not_finite_is_not_hidden(dtype, rows, bad):
+    w, _ = _matrix(dtype, rows, 896, 3)
+    x = torch.randn(896, device="cuda")
+    x[700] = bad
+    y = torch.zeros(rows, device="cuda")
+    L.check(L.lib().dooms_cuda_matvec(dtype, w.data_ptr(), x.data_ptr(), y.data_ptr(), None, rows, 896, 0, 0))
+    assert not bool(torch.isfinite(y).any()) or dtype == L.F16 and float(torch.isfinite(y).float().mean()) < 0.01      # (an f16 weight of zero times inf is NaN as well)
+
+
+@pytest.mark.parametrize("dtype", [L.F16, L.Q4_0, L.Q4_K, L.Q6_K])
+@pytest.mark.parametrize("gate", [False, True])
+@pytest.mark.parametrize("tokens,rows,cols", [(1, 128, 256), (63, 130, 512), (65, 896, 1024), (129, 896, 4864), (300, 1152, 768), (513, 300, 512)])
+def test_matmul_over_its_token_tiles(dtype, gate, tokens, rows, cols):
+    w, values = _matrix(dtype, rows, cols, 11)
+    w2, values2 = _matrix(dtype, rows, cols, 12)
+    x = torch.randn(tokens, cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(7)).half()
+    y = torch.zeros(tokens, rows, device="cuda")
+    L.check(L.lib().dooms_cuda_matmul(dtype, w.data_ptr(), w2.data_ptr() if gate else None, x.data_ptr(), y.data_ptr(), None, tokens, rows, cols, 0, 0))
+    L.check(L.lib().dooms_cuda_kernel_status(0, None))
+    half = [v.half().double() for v in (values, values2)]      # the tiles hold the weights rounded to f16
+    ref = x.double() @ half[0].T
+    if gate:
+        ref = torch.nn.functional.silu(ref) * (x.double() @ half[1].T)
+    # f16 products are exact in f32; the accumulator adds cols / 16 partial sums: 1e-5 covers 4864 of them (measured 6e-6), the gate's product twice that
+    assert rel_l2(y.cpu().numpy(), ref.cpu().numpy()) < (2e-5 if gate else 1e-5)
+
+
+@pytest.mark.parametrize("position", [126, 254, 1022])
+def test_positions_around_a_range_and_a_cluster(tmp_path, position):
+    """A step's ranges are 128 keys, the blocks of eight of them merge in shared memory: the logits after one position per call are a prompt's."""
+    spec = synth.tiny_spec(synth.pure(L.Q8_0), context_length=2048)
+    path = write(tmp_path, "ranges", spec, 21)
+    ids = [int(t) for t in synth.prompt_tokens(position + 6, spec.n_vocab, 22)]
+    dec = CudaLlamaDecoder.load(path, 1200, 512)
+    dec.eval_tokens(ids[:position])
+    steps = []
+    for t in ids[position:]:
+        dec.eval_tokens([t])
+        steps.append(np.asarray(dec.logits()))
+    for i in (1, 2, 5):
+        dec.reset()
+        dec.eval_tokens(ids[:position + i + 1])
+        assert rel_l2(steps[i], np.asarray(dec.logits())) < 3e-3      # the bound of a prompt in one call (its tiles round operands to f16)
