@@ -181,18 +181,71 @@ __device__ __forceinline__ void dequant_q4_K_group(const uint32_t (&w)[36], uint
     }
 }
 
-// Whole rows to f16, the value every tile of the fused kernel would hold (half(Q::elem)): one thread per 32 elements.
+// Eight consecutive elements (k0 a multiple of 8) of a row as f16, by the formats' own formulas: the values elem<DT> gives, with what the eight share read once.
 template <int DT>
-__global__ void __launch_bounds__(256) k_dequant_f16(const uint8_t * W, __half * out, int64_t rows, int cols) {
-    const int64_t units = rows * (cols / 32);
-    const int64_t RB = row_bytes_of(DT, cols);
-    for (int64_t u = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; u < units; u += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t r = u / (cols / 32);
-        const uint32_t k0 = uint32_t(u - r * (cols / 32)) * 32u;
-        uint4 v[4];
-        dequant32<DT>(W + r * RB, k0, v);
-        uint4 * dst = reinterpret_cast<uint4 *>(out + r * cols + k0);
-        dst[0] = v[0]; dst[1] = v[1]; dst[2] = v[2]; dst[3] = v[3];
+__device__ __forceinline__ uint4 dequant8(const uint8_t * row, uint32_t k0) {
+    float v[8];
+    if constexpr (DT == kQ4_0 || DT == kQ5_0 || DT == kQ8_0) {
+        const uint8_t * b = row + size_t(k0 / 32) * BlockInfo<DT>::bytes;
+        const float d = ld_half(b);
+        const uint32_t j = k0 & 31u;                              // 0, 8, 16 or 24: one nibble of eight bytes
+        if constexpr (DT == kQ8_0) {
+            const uint32_t w[2] = {ld_u32_b2(b + 2 + j), ld_u32_b2(b + 6 + j)};
+            #pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = __fmul_rn(d, float(int8_t(w[i / 4] >> (8 * (i % 4)))));
+        } else {
+            constexpr uint32_t QS = DT == kQ5_0 ? 6u : 2u;
+            const uint32_t sh = (j >> 4) * 4u, w[2] = {ld_u32_b2(b + QS + (j & 15u)) >> sh, ld_u32_b2(b + QS + 4 + (j & 15u)) >> sh};
+            const uint32_t qh = DT == kQ5_0 ? ld_u32_b2(b + 2) >> j : 0u;
+            #pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint32_t q = ((w[i / 4] >> (8 * (i % 4))) & 15u) | (((qh >> i) & 1u) << 4);
+                v[i] = __fmul_rn(d, float(int(q) - (DT == kQ5_0 ? 16 : 8)));
+            }
+        }
+    } else if constexpr (DT == kQ4_K) {
+        const uint8_t * b = row + size_t(k0 / 256) * 144;
+        const uint32_t j = k0 & 255u, c = j / 32;
+        float sc, m;
+        scale_min_k4(c, b + 4, sc, m);
+        const float ds = __fmul_rn(ld_half(b), sc), dm = __fmul_rn(ld_half(b + 2), m);
+        const uint8_t * qs = b + 16 + 32 * (c / 2) + (j & 31u);
+        const uint32_t sh = (c & 1u) * 4u, w[2] = {ld_u32_b2(qs) >> sh, ld_u32_b2(qs + 4) >> sh};
+        #pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = __fsub_rn(__fmul_rn(ds, float((w[i / 4] >> (8 * (i % 4))) & 15u)), dm);
+    } else if constexpr (DT == kQ6_K) {
+        const uint8_t * b = row + size_t(k0 / 256) * 210;
+        const uint32_t j = k0 & 255u, h = j / 128, k = (j & 127u) / 32, l = j & 31u;
+        const float ds = __fmul_rn(ld_half(b + 208), float(reinterpret_cast<const int8_t *>(b + 192)[8 * h + l / 16 + 2 * k]));
+        const uint8_t * ql = b + 64 * h + (k & 1u) * 32 + l, * qh = b + 128 + 32 * h + l;
+        const uint32_t sl = (k >> 1) * 4u, sh = 2u * k;
+        const uint32_t w[2] = {ld_u32_b2(ql) >> sl, ld_u32_b2(ql + 4) >> sl}, z[2] = {ld_u32_b2(qh) >> sh, ld_u32_b2(qh + 4) >> sh};
+        #pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t q = ((w[i / 4] >> (8 * (i % 4))) & 15u) | (((z[i / 4] >> (8 * (i % 4))) & 3u) << 4);
+            v[i] = __fmul_rn(ds, float(int(q) - 32));
+        }
+    } else {
+        #pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = elem<DT>(row, k0 + i);
+    }
+    uint32_t out[4];
+    #pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+        out[i] = *reinterpret_cast<const uint32_t *>(&h);
+    }
+    return make_uint4(out[0], out[1], out[2], out[3]);
+}
+
+// Whole rows to f16, the value every tile of the fused kernel would hold (half(Q::elem)). Bound by device memory (0.56 to 1.06 bytes in and 2 out per element): a
+// thread makes eight consecutive elements, so a warp reads and writes whole consecutive lines (one thread per 32 elements, 64 bytes apart in its stores and every
+// scale unpacked per element, ran at 1.2 TB/s on q4_K: 310 us for 5120 x 27648).
+template <int DT>
+__global__ void __launch_bounds__(256) k_dequant_f16(const uint8_t * W, __half * out, uint32_t units, uint32_t per_row, int64_t RB) {
+    for (uint32_t u = blockIdx.x * 256u + threadIdx.x; u < units; u += gridDim.x * 256u) {
+        const uint32_t r = u / per_row;
+        reinterpret_cast<uint4 *>(out)[u] = dequant8<DT>(W + int64_t(r) * RB, (u - r * per_row) * 8u);
     }
 }
 
@@ -582,8 +635,12 @@ cudaError_t launch_dt(const CUtensorMap & map, const CUtensorMap & wmap, const C
 
 template <int DT>
 cudaError_t dequant_rows(const void * W, void * out, int64_t rows, int64_t cols, cudaStream_t stream) {
-    const int64_t units = rows * (cols / 32);
-    k_dequant_f16<DT><<<unsigned(std::min<int64_t>((units + 255) / 256, sm_count() * 16)), 256, 0, stream>>>(static_cast<const uint8_t *>(W), static_cast<__half *>(out), rows, int(cols));
+    const int64_t per_row = cols / 8, RB = row_bytes_of(DT, cols), most = (int64_t(1) << 30) / per_row;      // (rows per launch: units are counted in 32 bits)
+    for (int64_t r0 = 0; r0 < rows; r0 += most) {
+        const uint32_t units = uint32_t(std::min(most, rows - r0) * per_row);
+        k_dequant_f16<DT><<<unsigned(std::min<int64_t>((units + 255) / 256, sm_count() * 32)), 256, 0, stream>>>(static_cast<const uint8_t *>(W) + r0 * RB,
+                                                                                                                static_cast<__half *>(out) + r0 * cols, units, uint32_t(per_row), RB);
+    }
     return cudaGetLastError();
 }
 cudaError_t dequant_rows_dt(int dt, const void * W, void * out, int64_t rows, int64_t cols, cudaStream_t stream) {
@@ -687,6 +744,9 @@ static int k_splits_of_rows16(int M, int64_t N, int64_t K, int most) {
     return best;
 }
 
+// q4_K gate / up pairs go over f16 rows from this many tokens on: unpacking q4_K in the producers costs 1535 us for 2048 tokens of 27648 x 5120, the product on rows
+// 1035 with 120 for writing them. (q4_0 unpacks cheaply: 465 us for 2048 tokens of 14336 x 4096 against 452 + 50, it stays with the producers.)
+constexpr int kGateRowsFrom = 512;
 static bool wide_rows(int dt, int64_t K, const void * W) { return (dt == kQ4_0 || dt == kQ4_K) && K % 256 == 0 && (reinterpret_cast<uintptr_t>(W) & 15u) == 0; }
 // Whether a product runs on f16 rows: f16 weights always (they are such rows); others from pre_from_tokens() tokens on (see launch_gemm_tc), and at any number of
 // tokens when the format has no wide producers: one element after another in every tile, they pay a memory latency per k step (17 us for the 14 steps of an
@@ -694,7 +754,7 @@ static bool wide_rows(int dt, int64_t K, const void * W) { return (dt == kQ4_0 |
 static bool on_rows16(int dt, const void * W, int M, int64_t N, int64_t K, bool gate, size_t w16_bytes) {
     if (dt == kF16) return (reinterpret_cast<uintptr_t>(W) & 15u) == 0;
     const bool wide = wide_rows(dt, K, W);
-    return w16_bytes >= size_t(N) * size_t(K) * 2 * (gate ? 2 : 1) && (wide ? M >= pre_from_tokens() && !gate : true);
+    return w16_bytes >= size_t(N) * size_t(K) * 2 * (gate ? 2 : 1) && (!wide || (gate ? dt == kQ4_K && M >= kGateRowsFrom : M >= pre_from_tokens()));
 }
 
 int gemm_tc_k_splits(int dt, const void * W, int M, int64_t N, int64_t K, size_t w16_bytes, int most) {
