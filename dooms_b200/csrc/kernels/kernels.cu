@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kNormThreads) k_rms_norm(float * x, const floa
             g[k] = i < E ? gamma[i] : 0.f;
         }
         if (n_shares > 0) {
-            #pragma unroll 4
+            #pragma unroll 8
             for (int z = 0; z < n_shares; z++) {
                 #pragma unroll
                 for (int k = 0; k < kNormMaxPerThread; k++) {
@@ -547,12 +547,16 @@ cudaError_t launch_rms_norm(const float * x, const float * gamma, float * out, v
                             const float * shares, int n_shares, int64_t share_stride) {
     if ((xq && (rows != 1 || E % 32 != 0)) || (n_shares > 0 && !shares)) return cudaErrorInvalidValue;
     float * const xw = const_cast<float *>(x);
-    if (rows >= 64 && E <= 256 * 4) {      // (few registers: the shares of four products are loaded together)
+    if (rows >= 64 && E <= 256 * 4) {      // (few registers: eight shares of an element are loaded together)
         return launch_pdl(k_rms_norm<256, 4>, dim3(rows), dim3(256), 0, stream, xw, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps,
                           shares, n_shares, share_stride);
     }
     if (rows >= 64 && E <= 256 * 16) {
         return launch_pdl(k_rms_norm<256, 16>, dim3(rows), dim3(256), 0, stream, xw, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps,
+                          shares, n_shares, share_stride);
+    }
+    if (E <= 1024) {
+        return launch_pdl(k_rms_norm<1024, 1>, dim3(rows), dim3(1024), 0, stream, xw, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps,
                           shares, n_shares, share_stride);
     }
     return launch_pdl(k_rms_norm<1024, 8>, dim3(rows), dim3(1024), 0, stream, xw, gamma, out, static_cast<__half *>(out16), static_cast<uint8_t *>(xq), E, eps,
