@@ -396,7 +396,7 @@ struct CudaLlamaDecoder::Impl {
     // otherwise, or when prefill_tile = 1 asks for the plain kernels.
     void prefill_attention(__half * kcl, __half * vcl, __half * out16, int M, const AttnShape & as) {
         if (cfg.prefill_tile != 1 && cuda::attention_flash_supported(as)) {
-            run("attention", [&] { return cuda::launch_attention_flash(qkv, kcl, vcl, attn + attn_pad, out16 ? out16 + attn_pad : nullptr, state, M, as, stream); });
+            run("attention", [&] { return cuda::launch_attention_flash(qkv, kcl, vcl, out16 ? nullptr : attn + attn_pad, out16 ? out16 + attn_pad : nullptr, state, M, as, pos + M, stream); });
         } else {
             run("attention", [&] { return cuda::launch_attention_prefill(qkv, kcl, vcl, attn + attn_pad, out16 ? out16 + attn_pad : nullptr, state, M, as, stream); });
         }

@@ -127,7 +127,7 @@ cudaError_t launch_attention_prefill(const float * qkv, const void * kc, const v
 // The same on the tensor cores (attention_flash.cu) for head_dim 64 or 128.
 bool attention_flash_supported(const AttnShape & s);
 cudaError_t launch_attention_flash(const float * qkv, const void * kc, const void * vc, float * out, void * out16, const DevState * st, int M, const AttnShape & s,
-                                   cudaStream_t stream);
+                                   int keys, cudaStream_t stream);      // keys: positions the last query sees (st->pos + M), for the choice of how the work is dealt
 
 // tokens[st->tok_out] = first index of the maximum of logits[0..n) (NaN never wins); the token also goes to host_tokens[st->tok_out] when that is set
 // (mapped pinned memory). With advance the state moves one decode step forward (pos, tok_in, tok_out += 1). part: argmax_blocks(n) x 2 words.
