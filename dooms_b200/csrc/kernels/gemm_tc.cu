@@ -70,6 +70,10 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The IEEE division has a branch in it for each of the 64 to 128 results a lane works on; __fdividef is within two ulp of it (the result is rounded to f16 next; against
+// the f64 product both give 2.3e-6 at K = 896, the accumulator's own error) and lets them overlap: 21.8 -> 17.7 us for 512 tokens of 4864 x 896.
+__device__ __forceinline__ float silu(float v) { return __fdividef(v, 1.f + expf(-v)); }
+
 // Polls the count of consumed steps (a word in shared memory that only grows) until it reaches `want`; bounded like mbar_wait.
 __device__ __forceinline__ bool wait_consumed(uint32_t addr, int want) {
     for (uint32_t i = 0; i < kMaxPolls; i++) {
@@ -499,7 +503,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
                         #pragma unroll
                         for (int j = 0; j < 32; j++) {
                             const float v = __uint_as_float(acc[j]);
-                            acc[j] = __float_as_uint(v / (1.f + expf(-v)) * __uint_as_float(acc2[j]));
+                            acc[j] = __float_as_uint(silu(v) * __uint_as_float(acc2[j]));
                         }
                     } else {
                         #pragma unroll
@@ -593,7 +597,7 @@ __global__ void __launch_bounds__(256) k_gate_up_combine(const float * shares, i
             u += __ldcg(mine + (int64_t(z) * 2 + 1) * plane + idx);
         }
         if (m0 + j < M && n0 + r < N) {
-            const float v = g / (1.f + expf(-g)) * u;
+            const float v = silu(g) * u;
             if (Y) Y[int64_t(m0 + j) * y_stride + n0 + r] = v;
             if (Y16) Y16[int64_t(m0 + j) * y16_stride + n0 + r] = __float2half_rn(v);
         }
@@ -699,7 +703,7 @@ static int pre_from_tokens() {
 constexpr int kMaxSplits = 32;
 static int64_t wave_cost(int64_t blocks, int64_t block_cycles) { return (blocks + sm_count() - 1) / sm_count() * block_cycles; }
 static int64_t step_cycles(int T, bool gate) { return gate ? (T == 64 ? 700 : T == 128 ? 800 : 1100) : (T == 64 ? 560 : T == 128 ? 610 : 840); }
-static int64_t fixed_cycles(int T, bool gate) { return gate ? (T == 64 ? 8000 : T == 128 ? 12500 : 24000) : (T == 64 ? 5500 : T == 128 ? 6300 : 8000); }
+static int64_t fixed_cycles(int T, bool gate) { return gate ? (T == 64 ? 6500 : T == 128 ? 9000 : 15000) : (T == 64 ? 5500 : T == 128 ? 6300 : 8000); }
 constexpr int64_t kPairStep = 1450, kPairFixed = 14000;      // a block of 256 weight rows x 256 tokens
 // One matrix, 256 tokens per block: the first token tiles run as blocks of 256 weight rows (two accumulators that share the token tile, which cuts what a block
 // pulls out of L2 per flop by a third), the rest as plain tiles, whichever mix takes the least time; the number of the former comes back.
@@ -745,7 +749,7 @@ static int k_splits_of_rows16(int M, int64_t N, int64_t K, int most) {
 }
 
 // q4_K gate / up pairs go over f16 rows from this many tokens on: unpacking q4_K in the producers costs 1535 us for 2048 tokens of 27648 x 5120, the product on rows
-// 1035 with 120 for writing them. (q4_0 unpacks cheaply: 465 us for 2048 tokens of 14336 x 4096 against 452 + 50, it stays with the producers.)
+// 985 with 120 for writing them. (q4_0 unpacks cheaply: 465 us for 2048 tokens of 14336 x 4096 against 427 + 50, it stays with the producers.)
 constexpr int kGateRowsFrom = 512;
 static bool wide_rows(int dt, int64_t K, const void * W) { return (dt == kQ4_0 || dt == kQ4_K) && K % 256 == 0 && (reinterpret_cast<uintptr_t>(W) & 15u) == 0; }
 // Whether a product runs on f16 rows: f16 weights always (they are such rows); others from pre_from_tokens() tokens on (see launch_gemm_tc), and at any number of
