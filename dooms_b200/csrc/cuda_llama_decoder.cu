@@ -321,7 +321,7 @@ struct CudaLlamaDecoder::Impl {
             return;
         }
         if (writes_x) link_ready = false;
-        if (w.dt == DType::Q6_K && cuda::gemv_q6_k_supported(w.ptr, w.rows, w.cols) && (!gamma || (in == x && cfg.n_embd % 32 == 0))) {
+        if (w.dt == DType::Q6_K && cuda::gemv_q6_k_supported(w.ptr, w.rows, w.cols) && (!gamma || (w.cols == cfg.n_embd && cfg.n_embd % 32 == 0))) {
             // the integer tensor-core kernel for q6_K works on the split input: left by the norm, or made by one small kernel
             if (gamma) {
                 norm(in, gamma, 1, true);
