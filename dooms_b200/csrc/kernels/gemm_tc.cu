@@ -2,8 +2,8 @@
 // shared memory and multiplied with tcgen05.mma, accumulators in tensor memory.
 //
 //   * One block of threads computes 128 weight rows x up to 256 tokens. The weight tile is the MMA's A operand (M = 128: one weight row per TMEM lane), the
-//     token tile its B operand (N = 128 or 256), both K-major f16 in the 128-byte swizzled layout; D[n][m] lives in 256 TMEM columns (gate/up: two
-//     accumulators, all 512 columns).
+//     token tile its B operand (N = 64, 128 or 256), both K-major f16 in the 128-byte swizzled layout; D[n][m] lives in as many TMEM columns (gate/up: two
+//     accumulators, twice as many).
 //   * Per 64-wide k step: the token tile (f16 activations written by the producing kernel) arrives by TMA (cp.async.bulk.tensor.2d, one block of threads per copy); 256
 //     producer threads read the weight rows' raw blocks from global memory (two threads per row; q4_0 rows in 144-byte groups of 16-byte loads), dequantize them to f16 exactly as the
 //     reference's tiles do (half(Q::elem), src/backend/metal/llama_kernels.h:1027-1035, 197) and store them swizzled; one thread issues the four k = 16
@@ -11,11 +11,11 @@
 //     hanging.
 //   * Epilogue: the producer warps read their TMEM lanes (tcgen05.ld 32x32b), add bias / the residual, or apply silu(gate) * up, and write coalesced
 //     rows of Y (f32) or of the f16 activation buffer the next GEMM reads.
-//   * From 128 tokens per call a matrix is first written out as f16 rows (k_dequant_f16, or a copy the caller keeps) and both operands arrive by TMA; the
-//     producer warps then only run the epilogue. On that route a block may take 256 weight rows (the second accumulator holds rows 128..255 against the
+//   * On the f16-row route (f16 weights; a copy the caller keeps; otherwise rows written by k_dequant_f16 first, see on_rows16) both operands arrive by TMA; the
+//     producer warps then only run the epilogue. There a block may take 256 weight rows (the second accumulator holds rows 128..255 against the
 //     same token tile), the first token tiles of a product running as such blocks and the rest as plain tiles, whichever split needs the fewest waves.
-//   * Two ways to deal a reduction over several blocks: a product of few weight rows against one token tile (a batched decode step) writes per-share sums
-//     that launch_add_shares adds in a fixed order; a fused gate / up product whose tiles leave a nearly empty last wave runs the leftover tiles that way
+//   * Two ways to deal a reduction over several blocks: a product of few tiles (a short chunk, a batched decode step) writes per-share sums
+//     that the next norm, or launch_add_shares, adds in a fixed order; a fused gate / up product whose tiles leave a nearly empty last wave runs the leftover tiles that way
 //     and k_gate_up_combine applies the epilogue.
 // Replaces matmul_bigq / matmul_gate_up_bigq and the dequant_half + matmul_big pair of the reference (llama_kernels.h:1320-1382, 1474-1480).
 #include <cuda.h>
