@@ -580,7 +580,9 @@ struct CudaLlamaDecoder::Impl {
         link_ready = false;      // x was just written by the embedding (or by the caller)
         // one position: its rotary angles are the same for every head of every layer
         cuda::DecodeLayersPlan * const one_launch = M == 1 ? fused_plan() : nullptr;
-        if (M == 1 && gqa) {
+        const bool have_table = rope_ready && !one_launch;
+        rope_ready = false;
+        if (M == 1 && gqa && !have_table) {
             run("rope_table", [&] { return cuda::launch_rope_table(state, inv_freq, rope_cs, cfg.head_dim, stream, one_launch ? cuda::decode_layers_barrier(one_launch) : nullptr); });
         }
         if (one_launch) {
@@ -693,6 +695,13 @@ struct CudaLlamaDecoder::Impl {
         }
     }
 
+    // The row of a step that forward() continues, with the rotary table of its position in the same launch.
+    bool rope_ready = false;
+    void embed_step(const int32_t * ids, const int32_t * index) {
+        const cuda::RopeTable rope{state, inv_freq, static_cast<float2 *>(rope_cs), cfg.head_dim / 2};
+        run("embed", [&] { return cuda::launch_embed(int(token_embd.dt), token_embd.ptr, ids, index, x, 1, cfg.n_embd, stream, gqa ? &rope : nullptr); });
+        rope_ready = gqa;
+    }
     void embed(const int32_t * ids, const int32_t * index, int rows) {
         run("embed", [&] { return cuda::launch_embed(int(token_embd.dt), token_embd.ptr, ids, index, x, rows, cfg.n_embd, stream); });
     }
@@ -700,7 +709,8 @@ struct CudaLlamaDecoder::Impl {
     // One chunk whose rows are in x (or whose ids are in in_tokens); the last row's greedy token lands in tokens[0] (run_chunk, metal_llama_decoder.mm:402-414).
     void run_chunk(int rows, bool from_tokens) {
         run("state", [&] { return cuda::launch_set_state(state, pos, 0, 0, stream); });
-        if (from_tokens) embed(in_tokens, nullptr, rows);
+        if (from_tokens && rows == 1) embed_step(in_tokens, nullptr);
+        else if (from_tokens) embed(in_tokens, nullptr, rows);
         forward(rows, false);
         pos += rows;
         has_pending = true;
@@ -708,7 +718,7 @@ struct CudaLlamaDecoder::Impl {
 
     // One decode step: embeds tokens[state->tok_in], writes its greedy token to tokens[state->tok_out], advances the state.
     void decode_step_launches() {
-        embed(tokens, &state->tok_in, 1);
+        embed_step(tokens, &state->tok_in);
         forward(1, true);
     }
 

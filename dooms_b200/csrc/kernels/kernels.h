@@ -36,7 +36,10 @@ __host__ __device__ inline float accumulate_base(float y, uint32_t flags) {
 cudaError_t launch_set_state(DevState * st, int32_t pos, int32_t tok_in, int32_t tok_out, cudaStream_t stream);
 
 // x[row][:] = table[ids[(index ? *index : 0) + row]][:], rows x E (embedq<Q>, llama_kernels.h:1289-1296).
-cudaError_t launch_embed(int dt, const void * table, const int32_t * ids, const int32_t * index, float * x, int rows, int E, cudaStream_t stream);
+// rope (optional, one row): launch_rope_table's output in the same launch.
+struct RopeTable { const DevState * st; const double * inv_freq; float2 * cs; int pairs; };
+cudaError_t launch_embed(int dt, const void * table, const int32_t * ids, const int32_t * index, float * x, int rows, int E, cudaStream_t stream,
+                         const RopeTable * rope = nullptr);
 
 // out[r][:] = x[r][:] * rsqrt(mean(x[r]^2) + eps) * gamma (norm_vec, llama_kernels.h:1272-1286). out16 (optional) also receives the rows as f16; xq
 // (optional, one row, E a multiple of 32) the row split for the staged q4_0 GEMV.
@@ -92,7 +95,7 @@ cudaError_t launch_attention_gqa(const float * qkv, void * kc, void * vc, float 
                                  int splits, const AttnShape & s, int * counters, float * out, void * xq, cudaStream_t stream,
                                  const void * rope_cs = nullptr,    // launch_rope_table's output for st->pos, used instead of computing the angles
                                  // the caller vouches that st->pos and the cache rows before it were final before this kernel could start: a launch_rope_table
-                                 // earlier in the stream orders them (its dependents start only after its own wait); rows may then be read before the wait. The value: the
+                                 // (or a launch_embed with its table) earlier in the stream orders them (its dependents start only after its own wait); rows may then be read before the wait. The value: the
                                  // positions the caches have room for.
                                  int cache_keys = 0,
                                  // ranges' blocks as clusters that merge in shared memory: for a kernel in front whose blocks leave room on the SMs (launch_gemv_short).
