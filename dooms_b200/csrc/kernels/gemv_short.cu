@@ -243,10 +243,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_gemv_short(const __grid_constan
     }
     cp_async_commit();
     for (int i = tid; i < ntm * kWarps * kTileRows; i += kThreads) partial[i] = 0.f;
-    const float bias = ((p.flags & kFlagBias) && tid < nrows) ? __ldg(q.bias + R0 + tid) : 0.f;
     float gm[kHeld];
     load_gains<kWarps>(p.in, gm);
     pdl_wait();
+    // The bias is a buffer of the caller's like x and y: the kernel in front may be the one that writes it.
+    const float bias = ((p.flags & kFlagBias) && tid < nrows) ? __ldcg(q.bias + R0 + tid) : 0.f;
     const float old = ((p.flags & kFlagAccumulate) && tid < nrows) ? __ldcg(q.y + R0 + tid) : 0.f;      // y is final here too: nobody else writes these rows
     prepare_input<HALF, kWarps>(p.in, gm, smem, red);
     if (p.in.ss && warp == 0) {

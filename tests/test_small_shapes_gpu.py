@@ -49,6 +49,26 @@ def test_matvec_of_small_and_tall_matrices(dtype, rows, cols):
 
 
 @pytest.mark.parametrize("dtype", SHORT_TYPES)
+def test_a_bias_that_the_call_before_writes(dtype):
+    """y1 = W1 x, then y2 = W2 x2 + y1 on the same stream: the second call may start early, but not read y1 before the first is done. W1 is the larger one, so the
+    second is waiting while y1 is being written; in between y1 holds NaN."""
+    w1, v1 = _matrix(dtype, 896, 4864, 31)
+    w2, v2 = _matrix(dtype, 896, 64, 32)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    x1, x2 = torch.randn(4864, device="cuda", generator=gen), torch.randn(64, device="cuda", generator=gen)
+    y1, y2 = torch.empty(896, device="cuda"), torch.empty(896, device="cuda")
+    ref = v1 @ x1.double() + v2 @ x2.double()
+    bound = _bound(dtype, v1, x1) + _bound(dtype, v2, x2) + 4 * U * (v1 @ x1.double()).abs() + 4 * U * ref.abs()
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(300):
+        y1.fill_(float("nan"))
+        L.check(L.lib().dooms_cuda_matvec(dtype, w1.data_ptr(), x1.data_ptr(), y1.data_ptr(), None, 896, 4864, 0, 0))
+        L.check(L.lib().dooms_cuda_matvec(dtype, w2.data_ptr(), x2.data_ptr(), y2.data_ptr(), y1.data_ptr(), 896, 64, 4, 0))
+        wrong += (~((y2.double() - ref).abs() <= bound)).sum()
+    assert int(wrong) == 0
+
+
+@pytest.mark.parametrize("dtype", SHORT_TYPES)
 @pytest.mark.parametrize("rows,cols", [(1, 64), (32, 896), (4864, 896), (33, 256)])
 def test_gate_up_of_small_matrices(dtype, rows, cols):
     wg, vg = _matrix(dtype, rows, cols, 1)
