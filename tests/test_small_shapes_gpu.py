@@ -113,6 +113,28 @@ def test_matmul_over_its_token_tiles(dtype, gate, tokens, rows, cols):
     assert rel_l2(y.cpu().numpy(), ref.cpu().numpy()) < (2e-5 if gate else 1e-5)
 
 
+@pytest.mark.parametrize("tokens", [64, 512])
+def test_silu_of_a_gate_up_product_is_the_divisions(tokens):
+    """One-hot tokens against weights that run through all finite f16 values, and an up matrix of ones: each result is silu of one value. It is
+    v / (1 + exp(-v)) in f32 with the division rounded to nearest, but for a last bit here and there; past exp(-v) = 2^126 it may be zero."""
+    v = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.float16)
+    v = v[torch.isfinite(v)]
+    w = v[:v.numel() // 64 * 64].view(-1, 64).cuda().contiguous()
+    ones = torch.ones_like(w)
+    x = torch.eye(64, dtype=torch.float16, device="cuda").repeat(tokens // 64, 1).contiguous()
+    y = torch.empty(tokens, w.shape[0], device="cuda")
+    L.check(L.lib().dooms_cuda_matmul(L.F16, w.data_ptr(), ones.data_ptr(), x.data_ptr(), y.data_ptr(), None, tokens, w.shape[0], 64, 0, 0))
+    L.check(L.lib().dooms_cuda_kernel_status(0, None))
+    got, wf = y.T.reshape(w.shape[0], tokens // 64, 64), w.float()
+    want = wf / (1 + torch.exp(-wf))
+    small = wf < -87
+    for t in range(tokens // 64):
+        g = got[:, t]
+        assert float((g - want)[small].abs().max()) < 1.1e-36
+        ulps = (g.view(torch.int32) - want.view(torch.int32)).abs()[~small]
+        assert int(ulps.max()) <= 1 and float((ulps > 0).float().mean()) < 0.01
+
+
 @pytest.mark.parametrize("position", [126, 254, 1022])
 def test_positions_around_a_range_and_a_cluster(tmp_path, position):
     """A step's ranges are 128 keys, the blocks of eight of them merge in shared memory: the logits after one position per call are a prompt's."""
