@@ -15,7 +15,9 @@ __device__ __forceinline__ void split_block(float v, int lane, int blk, int nb, 
     eb = max(eb, 30u);                                         // blocks below 2^-97 are treated as that small: their digits come out zero
     eb = min(eb, 250u);
     const float inv = __uint_as_float((279u - eb) << 23);      // 2^26 / s with s = 2^(eb - 126) > amax
-    int X = __float2int_rn(v * inv);
+    // Within 2^26 for a finite block (of values below 2^124), so the bounds touch infinities alone: they become +-(33 * 128^3 + 128), the digits +-33 and +-1 at the top of either pair, and their
+    // neighbours (below 2^97) zero.
+    int X = min(max(__float2int_rn(v * inv), -69206144), 69206144);
     int l[4];
     #pragma unroll
     for (int i = 0; i < 3; i++) { l[i] = ((X + 64) & 127) - 64; X = (X - l[i]) >> 7; }
@@ -26,9 +28,11 @@ __device__ __forceinline__ void split_block(float v, int lane, int blk, int nb, 
     for (int i = 0; i < 4; i++) dst[i * 32 + pos] = uint8_t(int8_t(l[i]));
     if (lane == 0) {
         float * sx = reinterpret_cast<float *>(xq + size_t(nb) * 128) + blk * 2;
-        const bool finite = amax < 0x7F800000u;                // a block with an infinity or a NaN in it makes every sum it enters NaN
-        sx[0] = __uint_as_float(finite ? (eb - 29u) << 23 : 0x7FC00000u);      // s * 2^-26 / 16: the weights carry a factor 16
-        sx[1] = __uint_as_float(finite ? (eb - 15u) << 23 : 0x7FC00000u);      // the same for the upper digit pair (x 2^14)
+        // A block that is not finite has its largest magnitude itself for a factor. An infinity: a row's sum is what the product with its weight is in f32, an infinity or
+        // (weight zero) NaN; of several in one block, the sign of their sum's. A NaN: every sum the block enters is NaN.
+        const bool finite = amax < 0x7F800000u;
+        sx[0] = __uint_as_float(finite ? (eb - 29u) << 23 : amax);      // s * 2^-26 / 16: the weights carry a factor 16
+        sx[1] = __uint_as_float(finite ? (eb - 15u) << 23 : amax);      // the same for the upper digit pair (x 2^14)
     }
 }
 

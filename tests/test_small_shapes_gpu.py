@@ -83,16 +83,22 @@ def test_gate_up_of_small_matrices(dtype, rows, cols):
     assert bool(((h.double() - ref).abs() <= 1.1 * bg * (u.abs() + bu) + g.abs() * bu + 16 * U * ref.abs() + 1e-30).all())
 
 
-@pytest.mark.parametrize("dtype", SHORT_TYPES)
+@pytest.mark.parametrize("dtype", SHORT_TYPES + [L.Q4_K, L.Q6_K])
 @pytest.mark.parametrize("rows", [64, 18977])
-@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
 def test_an_input_that_is_not_finite_is_not_hidden(dtype, rows, bad):
-    w, _ = _matrix(dtype, rows, 896, 3)
-    x = torch.randn(896, device="cuda")
+    """One such element: NaN everywhere; an infinity through the kernels of this file as in f32, +-inf by the sign of its weight and NaN where that is zero."""
+    cols = 1024 if dtype in (L.Q4_K, L.Q6_K) else 896
+    w, values = _matrix(dtype, rows, cols, 3)
+    x = torch.randn(cols, device="cuda")
     x[700] = bad
     y = torch.zeros(rows, device="cuda")
-    L.check(L.lib().dooms_cuda_matvec(dtype, w.data_ptr(), x.data_ptr(), y.data_ptr(), None, rows, 896, 0, 0))
-    assert not bool(torch.isfinite(y).any()) or dtype == L.F16 and float(torch.isfinite(y).float().mean()) < 0.01      # (an f16 weight of zero times inf is NaN as well)
+    L.check(L.lib().dooms_cuda_matvec(dtype, w.data_ptr(), x.data_ptr(), y.data_ptr(), None, rows, cols, 0, 0))
+    assert not bool(torch.isfinite(y).any())
+    want = values[:, 700] * bad
+    if np.isnan(bad) or dtype in SHORT_TYPES:
+        assert bool((torch.isnan(y) == torch.isnan(want)).all())
+        assert bool((torch.isnan(want) | (y.double() == want)).all())
 
 
 @pytest.mark.parametrize("dtype", [L.F16, L.Q4_0, L.Q4_K, L.Q6_K])
