@@ -137,7 +137,8 @@ __device__ __forceinline__ void attention_decode_body(const AttnDecodeParams & p
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, g = lane >> 2, t = lane & 3;
     const int G = p.s.n_head / p.s.n_head_kv;
     const bool fuse = p.inv_freq != nullptr;
-    const int pos = !fuse ? 0 : pp.b_slot ? row_pos : p.st->pos;
+    // (with cache_ready this is before the wait: the position is final in L2, but an SM may still hold the line of an earlier step in its L1)
+    const int pos = !fuse ? 0 : pp.b_slot ? row_pos : __ldcg(&p.st->pos);
     const int n_keys = p.n_keys_fixed > 0 ? p.n_keys_fixed : pos + 1;
     // Ranges of whole tiles, the same for every head. A range of two tiles takes as long as one of one tile (four warps each), so ranges are whole pairs, and only the first `used` of the p.splits ranges hold keys. The blocks of
     // the others leave at once and the merge reads `used` results (with one range there is nothing to merge): on the 0.5B shape, 2 key/value heads and so
