@@ -740,9 +740,12 @@ static int tokens_per_block(int M, int64_t N, int64_t K, bool gate, int splits) 
     for (int T : {128, 256}) if (tile_fits(T, M) && cut_cost(T, splits, M, N, K, gate) <= cut_cost(best, splits, M, N, K, gate)) best = T;
     return best;
 }
-static int k_splits_of_rows16(int M, int64_t N, int64_t K, int most) {
+static bool splits_off() {
     static const bool off = [] { const char * e = getenv("DOOMS_GEMM_SPLIT_K"); return e && *e == '0'; }();
-    if (off || K % kStepK != 0) return 1;
+    return off;
+}
+static int k_splits_of_rows16(int M, int64_t N, int64_t K, int most) {
+    if (splits_off() || K % kStepK != 0) return 1;
     const int ksteps = int(K / kStepK);
     int best = 1;
     int64_t best_cost = cut_cost(tokens_per_block(M, N, K, false, 1), 1, M, N, K, false);
@@ -770,7 +773,7 @@ static bool on_rows16(int dt, const void * W, int M, int64_t N, int64_t K, bool 
 
 int gemm_tc_k_splits(int dt, const void * W, int M, int64_t N, int64_t K, size_t w16_bytes, int most) {
     if (on_rows16(dt, W, M, N, K, false, w16_bytes)) return k_splits_of_rows16(M, N, K, most);
-    if (!wide_rows(dt, K, W)) return 1;
+    if (splits_off() || !wide_rows(dt, K, W)) return 1;
     // The wide producers: a block takes as long as its k steps (0.45 us each: the groups' loads are a chain of latencies), so a product of few row tiles is dealt over
     // the idle SMs in shares of whole 256-element groups.
     const int64_t tiles = (N + kRowsW - 1) / kRowsW * ((M + 255) / 256);
