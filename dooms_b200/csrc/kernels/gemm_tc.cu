@@ -771,6 +771,13 @@ static bool on_rows16(int dt, const void * W, int M, int64_t N, int64_t K, bool 
     return w16_bytes >= size_t(N) * size_t(K) * 2 * (gate ? 2 : 1) && (!wide || (gate ? dt == kQ4_K && M >= kGateRowsFrom : M >= pre_from_tokens()));
 }
 
+// Whether `units` units of the reduction make exactly k_splits shares, none of them empty: whoever adds the shares reads k_splits of them.
+static bool shares_fill(int64_t units, int k_splits) {
+    if (k_splits <= 1) return true;
+    const int64_t per = (units + k_splits - 1) / k_splits;
+    return k_splits <= kMaxSplits && k_splits <= units && (units + per - 1) / per == k_splits;
+}
+
 int gemm_tc_k_splits(int dt, const void * W, int M, int64_t N, int64_t K, size_t w16_bytes, int most) {
     if (on_rows16(dt, W, M, N, K, false, w16_bytes)) return k_splits_of_rows16(M, N, K, most);
     if (splits_off() || !wide_rows(dt, K, W)) return 1;
@@ -833,7 +840,7 @@ static cudaError_t launch_rows16(GemmTcParams p, const CUtensorMap & xmap, const
 cudaError_t launch_gemm_tc_rows16(const void * W16, const void * W2_16, const TensorMap * xmap, float * Y, void * Y16, const float * bias, int M, int64_t N, int64_t K,
                                   int64_t y_stride, int64_t y16_stride, uint32_t flags, int32_t * error, cudaStream_t stream, int k_splits, int64_t split_stride) {
     if (!W16 || N < 1 || K < kStepK || K % kStepK != 0 || M < 1 || (reinterpret_cast<uintptr_t>(W16) & 15u) || (reinterpret_cast<uintptr_t>(W2_16) & 15u)) return cudaErrorInvalidValue;
-    if (k_splits > 1 && (k_splits > kMaxSplits || W2_16 || !Y || Y16 || flags || split_stride < int64_t(M) * y_stride)) return cudaErrorInvalidValue;
+    if (!shares_fill(K / kStepK, k_splits) || (k_splits > 1 && (W2_16 || !Y || Y16 || flags || split_stride < int64_t(M) * y_stride))) return cudaErrorInvalidValue;
     GemmTcParams p{nullptr, nullptr, Y, static_cast<__half *>(Y16), bias, N, int(K), M, y_stride, y16_stride, flags, M > 128 ? 256 : 128, 0, 0, 0, 0, 0, 0, nullptr, error};
     return launch_rows16(p, *reinterpret_cast<const CUtensorMap *>(xmap), static_cast<const __half *>(W16), static_cast<const __half *>(W2_16), M, N, K, k_splits,
                          split_stride, stream);
@@ -848,22 +855,26 @@ cudaError_t launch_gemm_tc(int dt, const void * W, const void * W2, const Tensor
                            int64_t y_stride, int64_t y16_stride, uint32_t flags, int32_t * error, cudaStream_t stream, void * w16_scratch, size_t w16_bytes, int k_splits,
                            int64_t split_stride) {
     if (!gemm_tc_supported(dt, W, N, K) || M < 1) return cudaErrorInvalidValue;
-    if (k_splits > 1 && (k_splits > kMaxSplits || W2 || !Y || Y16 || flags || split_stride < int64_t(M) * y_stride)) return cudaErrorInvalidValue;
+    const bool gate = W2 != nullptr;
+    const bool rows16 = on_rows16(dt, W, M, N, K, gate, w16_scratch ? w16_bytes : 0) && (dt != kF16 || (reinterpret_cast<uintptr_t>(W2) & 15u) == 0);
+    if (k_splits > 1) {      // shares are of whole k steps on f16 rows, of whole 256-element groups from the wide producers; no other route deals a reduction
+        if (gate || !Y || Y16 || flags || split_stride < int64_t(M) * y_stride || !(rows16 || wide_rows(dt, K, W))) return cudaErrorInvalidValue;
+        if (!shares_fill(rows16 ? K / kStepK : K / 256, k_splits)) return cudaErrorInvalidValue;
+    }
     GemmTcParams p{static_cast<const uint8_t *>(W), static_cast<const uint8_t *>(W2), Y, static_cast<__half *>(Y16), bias, N, int(K), M, y_stride, y16_stride,
                    flags, M > 128 ? 256 : M > 64 ? 128 : 64, 0, 0, 0, 0, 0, 0, nullptr, error};
     p.wide = wide_rows(dt, K, W) && (!W2 || wide_rows(dt, K, W2)) ? 1 : 0;
     const CUtensorMap & map = *reinterpret_cast<const CUtensorMap *>(xmap);
-    const bool gate = W2 != nullptr;
     // Many tokens: dequantize the matrix once to f16 rows and let TMA feed both operands (the reference does the same from 320 tokens on,
     // metal_llama_decoder.mm:31); otherwise every token tile would redo the dequantization in its producer warps.
     // (from 128 tokens: a batched decode step of 256 rows on the 0.5B shape measured 6.4 ms with the weights dequantized by each block's producer warps
     // and 5.5 ms from f16 rows; with few blocks per matrix the producers' loads are a chain of memory latencies)
     // Measured on the 8B shapes: q4_0 / q4_K gate/up is faster fused (875 against 836 TFLOP/s: no f16 copy to write and read), everything else is faster
     // or much faster from f16 rows (ffn_down 961 against 925; q6_K 754 against 83).
-    if (dt == kF16 && on_rows16(dt, W, M, N, K, gate, 0) && (!W2 || (reinterpret_cast<uintptr_t>(W2) & 15u) == 0)) {
+    if (dt == kF16 && rows16) {
         return launch_rows16(p, map, static_cast<const __half *>(W), static_cast<const __half *>(W2), M, N, K, k_splits, split_stride, stream);
     }
-    if (dt != kF16 && w16_scratch && on_rows16(dt, W, M, N, K, gate, w16_bytes)) {
+    if (rows16) {
         __half * w16 = static_cast<__half *>(w16_scratch);
         cudaError_t e = dequant_rows_dt(dt, W, w16, N, K, stream);
         if (e == cudaSuccess && gate) e = dequant_rows_dt(dt, W2, w16 + size_t(N) * size_t(K), N, K, stream);
@@ -871,7 +882,6 @@ cudaError_t launch_gemm_tc(int dt, const void * W, const void * W2, const Tensor
         return launch_rows16(p, map, w16, gate ? w16 + size_t(N) * size_t(K) : nullptr, M, N, K, k_splits, split_stride, stream);
     }
     if (k_splits > 1) {      // (wide producers, see gemm_tc_k_splits)
-        if (!p.wide) return cudaErrorInvalidValue;
         const int groups = int(K / 256);
         p.ks_per = (groups + k_splits - 1) / k_splits * 4;
         p.split_stride = split_stride;

@@ -47,6 +47,20 @@ def fills(units, k):
     return -(-units // per) == k
 
 
+def test_a_count_of_shares_that_the_reduction_does_not_divide_into_is_refused(entries):
+    """A share that no block writes would be added by the norm all the same."""
+    if torch.cuda.is_available():
+        pytest.skip("the refusal comes before any use of the device; where there is one, nothing is tried that might be launched")
+    for units in (9, 36, 76, 224):
+        for k in range(2, 41):
+            if k > 32 or not fills(units, k):
+                assert entries.kernel_gemm_refuses(L.F16, 1, 256, units * 64, k), (units, k)
+                assert entries.kernel_gemm_refuses(L.F16, 0, 256, units * 64, k), (units, k)
+                assert entries.kernel_gemm_refuses(L.Q4_0, 0, 256, units * 256, k), (units, k)
+                assert entries.kernel_gemm_refuses(L.Q4_K, 0, 256, units * 256, k), (units, k)
+    assert entries.kernel_gemm_refuses(L.Q5_0, 0, 256, 2048, 2)      # no scratch for its rows: that route deals nothing
+
+
 def test_planned_counts_of_shares_divide_the_reduction(entries):
     for M in (1, 2, 16, 64, 65, 128, 300, 512, 2048):
         for N, K in ((896, 896), (896, 4864), (256, 2304), (4096, 4096), (4096, 14336), (5120, 27648), (64, 64), (130, 320)):
