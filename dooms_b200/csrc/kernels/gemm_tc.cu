@@ -697,9 +697,9 @@ cudaError_t make_rows_map(TensorMap * out, const void * base, int64_t rows, int6
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// The f16-row path is taken from this many tokens on (see launch_gemm_tc).
-static int pre_from_tokens() {
-    static const int v = [] { const char * e = getenv("DOOMS_GEMM_PRE_FROM"); return e ? atoi(e) : 128; }();
+// The token count from which quantized projections run on f16 rows, when the environment sets one; -1: by on_rows16's own rules.
+static int rows16_from() {
+    static const int v = [] { const char * e = getenv("DOOMS_GEMM_PRE_FROM"); return e ? std::max(0, atoi(e)) : -1; }();
     return v;
 }
 
@@ -762,13 +762,17 @@ static int k_splits_of_rows16(int M, int64_t N, int64_t K, int most) {
 // 985 with 120 for writing them. (q4_0 unpacks cheaply: 465 us for 2048 tokens of 14336 x 4096 against 427 + 50, it stays with the producers.)
 constexpr int kGateRowsFrom = 512;
 static bool wide_rows(int dt, int64_t K, const void * W) { return (dt == kQ4_0 || dt == kQ4_K) && K % 256 == 0 && (reinterpret_cast<uintptr_t>(W) & 15u) == 0; }
-// Whether a product runs on f16 rows: f16 weights always (they are such rows); others from pre_from_tokens() tokens on (see launch_gemm_tc), and at any number of
-// tokens when the format has no wide producers: one element after another in every tile, they pay a memory latency per k step (17 us for the 14 steps of an
-// 896-wide product, 37 us for 76), the pass that writes the rows 3 to 6 us.
+// Whether a product runs on f16 rows: f16 weights always (they are such rows); rows with wide producers from kRowsFrom tokens on (see launch_gemm_tc), their gate / up
+// pairs as above; the other formats at any number of tokens: one element after another in every tile, their producers pay a memory latency per k step (17 us for
+// the 14 steps of an 896-wide product, 37 us for 76), the pass that writes the rows 3 to 6 us. A count set in the environment stands for all of these, gate / up
+// pairs with wide producers excepted.
+constexpr int kRowsFrom = 128;
 static bool on_rows16(int dt, const void * W, int M, int64_t N, int64_t K, bool gate, size_t w16_bytes) {
     if (dt == kF16) return (reinterpret_cast<uintptr_t>(W) & 15u) == 0;
+    if (w16_bytes < size_t(N) * size_t(K) * 2 * (gate ? 2 : 1)) return false;
     const bool wide = wide_rows(dt, K, W);
-    return w16_bytes >= size_t(N) * size_t(K) * 2 * (gate ? 2 : 1) && (!wide || (gate ? dt == kQ4_K && M >= kGateRowsFrom : M >= pre_from_tokens()));
+    if (rows16_from() >= 0) return M >= rows16_from() && !(wide && gate);
+    return !wide || (gate ? dt == kQ4_K && M >= kGateRowsFrom : M >= kRowsFrom);
 }
 
 // Whether `units` units of the reduction make exactly k_splits shares, none of them empty: whoever adds the shares reads k_splits of them.

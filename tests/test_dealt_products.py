@@ -86,3 +86,5 @@ def test_the_switches_of_dealt_products(entries):
     assert all(k > 1 for k in plain.values()), plain
     off = planned({"DOOMS_GEMM_SPLIT_K": "0"})
     assert set(off.values()) == {1}, off
+    never = planned({"DOOMS_GEMM_PRE_FROM": "100000"})      # no quantized product on f16 rows: q5_0 and q8_0 have no other route that deals one
+    assert never[L.Q8_0, 45] == never[L.Q5_0, 300] == 1 and never[L.Q4_0, 45] == plain[L.Q4_0, 45] and never[L.F16, 45] == plain[L.F16, 45], never
