@@ -1173,15 +1173,6 @@ Result<std::unique_ptr<CudaLlamaDecoder>> CudaLlamaDecoder::create(const LlamaDe
     // a decode step over several slots needs the tensor-core chunk path, the grouped-query attention kernel and the whole model on this GPU
     m.max_rows = (n_seq > 1 && tp == 1 && m.tc_capable && m.gqa && cuda::gemm_tc_supported(int(m.output.dt), m.output.ptr, m.output.rows, m.output.cols))
                      ? std::min<int32_t>({n_seq, c.n_batch, 1024}) : 0;
-    if (m.tc_capable && tp == 1) {
-        // room for the shares of a reduction: what a batched step may want, at least 24 MB (ten shares of a 512-token chunk of 896-wide rows, eleven of a
-        // 128-token one of 4096); optional, without it no product is dealt
-        m.share_floats = std::max<size_t>(size_t(6) << 20, size_t(Impl::kMaxShares) * size_t(m.max_rows) * size_t(E));
-        if (cudaMalloc(reinterpret_cast<void **>(&m.shares), m.share_floats * sizeof(float)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            m.shares = nullptr;
-        }
-    }
     if (m.max_rows > 0) {
         const size_t R = size_t(m.max_rows);
         // Rows attend over very different lengths (a fresh sequence beside one at the end of its context), so a row is cut into ranges of a fixed number of
@@ -1233,6 +1224,17 @@ Result<std::unique_ptr<CudaLlamaDecoder>> CudaLlamaDecoder::create(const LlamaDe
             cudaHostAlloc(reinterpret_cast<void **>(&m.h_out), size_t(Impl::kMaxBatchSteps) * R * sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess) {
             (void)cudaGetLastError();
             return resource_exhausted("could not allocate pinned host memory for the batched decode step");
+        }
+    }
+    if (m.tc_capable && tp == 1) {
+        // Room for the shares of a reduction: what a batched step may want, and for chunks up to 24 MB (ten shares of a 512-token chunk of 896-wide rows, eleven of a
+        // 128-token one of 4096), less where n_batch rows cannot use that much. Optional, without it no product is dealt; so it comes after all that is not.
+        const size_t most = size_t(Impl::kMaxShares) * size_t(E);
+        const size_t chunk = c.prefill_tile == 1 ? 0 : std::min(size_t(6) << 20, most * B);
+        m.share_floats = std::max(chunk, most * size_t(m.max_rows));
+        if (m.share_floats > 0 && cudaMalloc(reinterpret_cast<void **>(&m.shares), m.share_floats * sizeof(float)) != cudaSuccess) {
+            (void)cudaGetLastError();
+            m.shares = nullptr;
         }
     }
     if (tp > 1) {

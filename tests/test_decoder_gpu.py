@@ -97,6 +97,20 @@ def test_longer_prompts_in_one_call(model_dir, plan):
         check_long_prompt(dec, path, 400, prompt, want)
 
 
+@pytest.mark.parametrize("n_batch,kw", [(8, {}), (64, {"prefill_tile": 1})])
+def test_a_decoder_of_small_chunks_holds_little_memory(model_dir, n_batch, kw):
+    """The tiny model is 4 MB and its buffers less; room for dealt reductions is held for the chunks there can be, and not where no chunk takes that path."""
+    import torch
+    path = write(model_dir, "tiny_memory", synth.tiny_spec(QUANT_PLANS["q4_0"]), 1)
+    CudaLlamaDecoder.load(path, 128, n_batch, **kw).close()      # what a first decoder makes the driver load stays
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    dec = CudaLlamaDecoder.load(path, 128, n_batch, **kw)
+    held = before - torch.cuda.mem_get_info()[0]
+    dec.close()
+    assert held < 20 << 20, held
+
+
 @pytest.mark.parametrize("qwen", [False, True])
 def test_long_context_decode_matches_the_oracle(model_dir, qwen):
     """Decode steps from position 520 on, where the cache is attended in several splits (test_metal_llama_decoder.cpp:467-495); head_dim 64."""
