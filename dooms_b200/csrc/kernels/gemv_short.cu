@@ -37,6 +37,7 @@ constexpr int kTileRows = 16;
 constexpr int kHeld = 8;                       // input blocks a warp keeps in registers while it normalizes: rows of up to 2048 make one pass
 constexpr int64_t kOwnNorm = int64_t(kHeld) * kWarps * 32;
 constexpr int kMaxRows = 64;                   // rows per block
+template <bool HALF> constexpr int kPerSm = HALF ? 3 : 2;      // blocks per SM that the registers are to allow (72 and 90 a thread)
 constexpr size_t kSmemLimit = 92 * 1024;       // two blocks per SM always fit, whatever kernel they belong to
 
 struct Input {
@@ -214,7 +215,7 @@ __device__ __forceinline__ void unit_dot(int dt, const uint8_t * smem, uint32_t 
 
 // HALF: f16 weights, the input as f32 in shared memory; otherwise block formats and the input as digits.
 template <bool HALF>
-__global__ void __launch_bounds__(kThreads, 2) k_gemv_short(const __grid_constant__ ShortParams p) {
+__global__ void __launch_bounds__(kThreads, kPerSm<HALF>) k_gemv_short(const __grid_constant__ ShortParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float red[kWarps];
     __shared__ float norm_scale;
@@ -430,7 +431,9 @@ Plan plan_rows(int dt, int64_t rows, int64_t cols, int nmat, int rpb) {
 }
 
 // Every block has to be resident at once with room beside it (the early start is the point), so a matrix is short when its share per SM, in one to three
-// blocks, fits. Rows per block: an equal share per SM, in whole 16-row tiles above 8 rows; whole 32-row groups when the results are to be split.
+// blocks, fits. Rows per block: an equal share per SM, in whole 16-row tiles above 8 rows; whole 32-row groups when the results are to be split. A gate / up
+// pair that does not fit so is halved until it does, and a half need not be whole tiles: 4864 x 896 in f16 goes from 48 rows to 24 and 12, at most 36 an SM,
+// where blocks of 16 would make it 48.
 // all_rows: the rows of all parts of the launch.
 Plan plan_for(int dt, int64_t rows, int64_t all_rows, int64_t cols, int nmat, bool split_out) {
     if (!takes_type(dt) || rows < 1 || cols < 64 || cols % 64 != 0 || cols > 65536 || all_rows > int64_t(3) * sm_count() * kMaxRows) return Plan{};
@@ -445,7 +448,11 @@ Plan plan_for(int dt, int64_t rows, int64_t all_rows, int64_t cols, int nmat, bo
         if (pl.ok || rpb <= 8 || nmat == 1) return pl;
     }
 }
-bool fits(const Plan & pl) { return pl.ok && int64_t(pl.blocks) <= int64_t(sm_count()) * std::min<int64_t>(3, int64_t((224 * 1024) / (pl.smem + 1024))); }
+// All blocks of the launch on the GPU at once, by shared memory and by registers.
+bool fits(int dt, const Plan & pl) {
+    const int64_t per_sm = std::min<int64_t>(dt == kF16 ? kPerSm<true> : kPerSm<false>, int64_t((224 * 1024) / (pl.smem + 1024)));
+    return pl.ok && int64_t(pl.blocks) <= int64_t(sm_count()) * per_sm;
+}
 
 // The longest chunk that leaves three stages a warp (two where no chunk does): fewer, longer copies per unit, and 2 x 16 of them in flight per SM.
 TallPlan tall_plan(int dt, int64_t rows, int64_t cols) {
@@ -473,7 +480,7 @@ TallPlan tall_plan(int dt, int64_t rows, int64_t cols) {
 
 bool gemv_short_own_norm(int64_t cols) { return cols <= kOwnNorm; }
 bool gemv_short_supported(int dt, const void * W, int64_t rows, int64_t cols, int nmat, bool split_out, int64_t all_rows) {
-    return (reinterpret_cast<uintptr_t>(W) & 15u) == 0 && fits(plan_for(dt, rows, all_rows > 0 ? all_rows : rows, cols, nmat, split_out));
+    return (reinterpret_cast<uintptr_t>(W) & 15u) == 0 && fits(dt, plan_for(dt, rows, all_rows > 0 ? all_rows : rows, cols, nmat, split_out));
 }
 
 cudaError_t launch_gemv_short(const ShortMatrix * mats, int n, const void * xq, const float * x, const float * gamma, float eps, int64_t cols, uint32_t flags,

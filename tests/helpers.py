@@ -60,3 +60,20 @@ def collect(dec, n: int, depth: int) -> list[int]:
     got: list[int] = []
     dec.generate(n, depth, lambda tok: got.append(tok) or True)
     return got
+
+
+def launched(call) -> list[tuple[str, list[int]]]:
+    """(name, grid) of the kernels that call() launches, in order, as the CUDA profiler lists them; empty where it is not available."""
+    import json
+    import tempfile
+
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    with tempfile.NamedTemporaryFile(suffix=".json") as f:
+        prof.export_chrome_trace(f.name)
+        events = [e for e in json.load(open(f.name))["traceEvents"] if e.get("cat") == "kernel"]
+    return [(e["name"], list(e["args"]["grid"])) for e in sorted(events, key=lambda e: e["ts"])]

@@ -7,7 +7,7 @@ import pytest
 
 from dooms_b200 import CudaLlamaDecoder, synth
 from dooms_b200 import _lib as L
-from helpers import rel_l2, write
+from helpers import launched, rel_l2, write
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -35,14 +35,17 @@ def _bound(dtype, values, x):
 
 
 @pytest.mark.parametrize("dtype", SHORT_TYPES)
-@pytest.mark.parametrize("rows,cols", [(1, 64), (7, 896), (8, 896), (9, 896), (149, 896), (896, 4864), (1153, 896), (18945, 128), (18977, 896)])
+@pytest.mark.parametrize("rows,cols", [(1, 64), (7, 896), (8, 896), (9, 896), (149, 896), (896, 4864), (1153, 896), (18945, 128), (18977, 896), (28417, 128), (28431, 896), (28417, 4096)])
 def test_matvec_of_small_and_tall_matrices(dtype, rows, cols):
     w, values = _matrix(dtype, rows, cols, rows + cols)
     gen = torch.Generator(device="cuda").manual_seed(5)
     x = torch.randn(cols, device="cuda", generator=gen)
     bias = torch.randn(rows, device="cuda", generator=gen)
     y = torch.full((rows,), 0.5, device="cuda")
-    L.check(L.lib().dooms_cuda_matvec(dtype, w.data_ptr(), x.data_ptr(), y.data_ptr(), bias.data_ptr(), rows, cols, 2 | 4, 0))      # y += W x + bias
+    names = launched(lambda: L.check(L.lib().dooms_cuda_matvec(dtype, w.data_ptr(), x.data_ptr(), y.data_ptr(), bias.data_ptr(), rows, cols, 2 | 4, 0)))      # y += W x + bias
+    # blocks of up to 64 rows, two (f16: three) on each of 148 SMs, 92 KB each at most (64 f16 rows of 896 are more)
+    tall = rows > (3 if dtype == L.F16 else 2) * 148 * 64 or (dtype == L.F16 and (rows, cols) == (18977, 896))
+    assert not names or ("k_gemv_tall" if tall else "k_gemv_short") in names[0][0]
     ref = values @ x.double()
     err = (y.double() - (ref + bias.double() + 0.5)).abs()
     assert bool((err <= _bound(dtype, values, x) + 4 * U * (ref.abs() + bias.abs().double() + 1)).all())
