@@ -38,7 +38,7 @@ constexpr int kHeld = 8;                       // input blocks a warp keeps in r
 constexpr int64_t kOwnNorm = int64_t(kHeld) * kWarps * 32;
 constexpr int kMaxRows = 64;                   // rows per block
 template <bool HALF> constexpr int kPerSm = HALF ? 3 : 2;      // blocks per SM that the registers are to allow (72 and 90 a thread)
-constexpr size_t kSmemLimit = 92 * 1024;       // two blocks per SM always fit, whatever kernel they belong to
+constexpr size_t kSmemLimit = 92 * 1024;       // two blocks per SM always fit, whatever kernel they belong to; the 8B attn_output's share (see plan_for)
 
 struct Input {
     const uint8_t * xq;      // the split input, or
@@ -441,8 +441,10 @@ Plan plan_for(int dt, int64_t rows, int64_t all_rows, int64_t cols, int nmat, bo
     const int sms = sm_count();
     int rpb = int((all_rows + sms - 1) / sms);
     if (rpb > 8) rpb = std::min(kMaxRows, (rpb + kTileRows - 1) / kTileRows * kTileRows);
-    // A gate / up pair may take up to three smaller blocks per SM. A plain projection that does not fit one per SM is left to the ring kernels: the 8B shape's qkv and
-    // attn_output, two and three blocks per SM here, made no difference after a prompt of 2048 tokens and cost 0.8 of 84.0 ms at a short one.
+    // A gate / up pair may take up to three smaller blocks per SM. A plain projection that does not fit one per SM is left to the ring kernels (the 8B shape's qkv: two
+    // and three blocks per SM here made no difference after a prompt of 2048 tokens and cost 0.8 of 84.0 ms at a short one). The 8B attn_output does fit: 32 rows of
+    // 4096 in q4_0 and their input are kSmemLimit to the byte. Its gate / up then normalizes the residual row in every block, where a ring kernel would have left it
+    // normalized and split (GemvNormLink): 37 + 48 tokens take 80.4 ms either way.
     for (;; rpb /= 2) {
         const Plan pl = plan_rows(dt, rows, cols, nmat, rpb);
         if (pl.ok || rpb <= 8 || nmat == 1) return pl;

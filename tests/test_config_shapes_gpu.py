@@ -29,7 +29,7 @@ from dooms_b200 import CudaLlamaDecoder, synth
 from oracle import binding as ob
 from oracle.streaming import StreamingOracle
 
-from helpers import rel_l2
+from helpers import launched, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -147,3 +147,31 @@ def test_token_by_token_matches_the_exact_checker_at_the_half_billion_shape():
     assert err < 1e-4 and within(got, want), err
     assert dec.pending_token() == ob.argmax(want)
     dec.close()
+
+
+def kernel_names(call):
+    import re
+    return [re.search(r"k_\w+", n).group(0) if "k_" in n else n for n, _ in launched(call)]
+
+
+@pytest.mark.parametrize("config,n_layer", [(0, 2), (1, 2), (2, 2), (3, 4)])
+def test_which_kernels_a_step_of_a_configuration_runs(config, n_layer):
+    """The dispatch rules at the configurations' shapes: qkv, attention, attn_output, gate / up and ffn_down of an even and of an odd layer, and the output matrix."""
+    path, _ = model_path(config, n_layer)
+    dec = CudaLlamaDecoder.load(path, 256, 64)
+    dec.eval_tokens([1, 2, 3])
+    got = kernel_names(lambda: dec.eval_tokens([4]))
+    dec.close()
+    if not got:
+        pytest.skip("the profiler lists no kernels here")
+    short = ["k_gemv_short", "k_attention_decode", "k_gemv_short", "k_gemv_short"]
+    ring = ["k_gemv_q4_0", "k_attention_decode", "k_gemv_q4_0", "k_gemv_q4_0"]
+    mixed = ["k_gemv_q4_0", "k_attention_decode", "k_gemv_short", "k_gemv_q4_0", "k_gemv_q4_0"]      # the 8B shape's attn_output fits one small block per SM
+    even, odd, output = {
+        0: (short + ["k_gemv_short"], short + ["k_gemv_short"], ["k_gemv_tall"]),
+        1: (short + ["k_gemv_q6_k"], short + ["k_gemv_q4_0"], ["k_gemv_tall"]),      # ffn_down q6_K and q4_K in turn
+        2: (mixed, mixed, ["k_gemv_tall"]),
+        3: (["k_gemv_q4_0", "k_gemv_q4_0", "k_rms_norm", "k_gemv_q6_k"] + ring[1:] + ["k_gemv_q6_k"], ring + ["k_gemv_q4_0"], ["k_rms_norm", "k_gemv_q6_k"]),
+    }[config]
+    want = ["k_set_state", "k_embed"] + [k for l in range(n_layer) for k in (even, odd)[l % 2]] + output + ["k_argmax_part", "k_argmax_final"]
+    assert got == want, got
