@@ -9,6 +9,8 @@ from dooms_b200 import _lib as L
 from dooms_b200.quantize import quantize
 from oracle import binding as ob
 
+from helpers import launched
+
 pytestmark = pytest.mark.gpu
 
 MATRIX_TYPES = [L.F16, L.Q4_0, L.Q5_0, L.Q8_0, L.Q4_K, L.Q6_K]
@@ -85,6 +87,58 @@ def test_matvec_matches_the_oracle(dtype, shape):
         assert np.all(np.abs(got - want) <= 2e-6 * scale + 1e-6 * np.abs(want) + 1e-30), (flags, np.abs(got - want).max())
 
 
+def taken_by(kernel, call):
+    """call() launches this kernel (where the profiler can tell): a rule that moves a shape elsewhere may not leave its old kernel untested."""
+    names = [n for n, _ in launched(call)]
+    assert not names or any(kernel in n for n in names), names
+
+
+# shapes whose share per SM is too large for the small-matrix kernel: the ring kernels, with ragged last tiles and blocks of unequal rows
+RING_SHAPES = [(L.Q4_0, (6145, 4096), "k_gemv_q4_0"), (L.Q4_0, (4097, 14336), "k_gemv_q4_0"), (L.Q4_0, (9001, 4160), "k_gemv_q4_0"), (L.Q4_K, (4097, 4096), "k_gemv_q4_0"), (L.Q6_K, (5121, 4096), "k_gemv_q6_k"),
+               (L.Q5_0, (4097, 4096), "k_gemv_blocks"), (L.Q8_0, (4097, 4096), "k_gemv_blocks"), (L.F16, (4097, 4096), "k_gemv_blocks"), (L.Q8_0, (4103, 2080), "k_gemv_blocks")]
+
+
+@pytest.mark.parametrize("dtype,shape,kernel", RING_SHAPES)
+def test_matvec_of_matrices_that_fill_the_gpu(dtype, shape, kernel):
+    rows, cols = shape
+    blocks = random_blocks(dtype, rows, cols, 12)
+    g = np.random.default_rng(6)
+    x, bias, y0 = (g.standard_normal(n).astype(np.float32) for n in (cols, rows, rows))
+    d_w, d_x, d_b = dev(blocks), dev(x), dev(bias)
+    d_v = torch.empty(rows, cols, device="cuda")          # (dequantization is held to the oracle's bits above)
+    L.check(L.lib().dooms_cuda_dequantize(dtype, d_w.data_ptr(), rows, cols, d_v.data_ptr(), None))
+    base = (d_v.double() @ d_x.double()).cpu().numpy()
+    scale = (d_v.double().abs() @ d_x.double().abs()).cpu().numpy()
+    for flags, want in ((0, base), (4, base + bias), (2, base + y0), (6, base + bias + y0)):
+        d_y = dev(y0.copy())
+        call = lambda: L.check(L.lib().dooms_cuda_matvec(dtype, d_w.data_ptr(), d_x.data_ptr(), d_y.data_ptr(), d_b.data_ptr(), rows, cols, flags, None))
+        taken_by(kernel, call) if flags == 6 else call()
+        torch.cuda.synchronize()
+        got = d_y.cpu().numpy().astype(np.float64)
+        assert np.all(np.abs(got - want) <= 2e-6 * scale + 1e-6 * np.abs(want) + 1e-30), (flags, np.abs(got - want).max())
+    L.check(L.lib().dooms_cuda_kernel_status(None, None))
+
+
+@pytest.mark.parametrize("dtype,shape,kernel", [(L.Q4_0, (4865, 4096), "k_gemv_q4_0"), (L.Q4_K, (4865, 4096), "k_gemv_q4_0"), (L.Q5_0, (4865, 4096), "k_gemv_blocks"),
+                                                (L.Q8_0, (4865, 4096), "k_gemv_blocks"), (L.F16, (4865, 4096), "k_gemv_blocks")])
+def test_gate_up_of_matrices_that_fill_the_gpu(dtype, shape, kernel):
+    rows, cols = shape
+    d_g, d_u = dev(random_blocks(dtype, rows, cols, 1)), dev(random_blocks(dtype, rows, cols, 2))
+    d_x = dev(np.random.default_rng(3).standard_normal(cols).astype(np.float32) * np.float32(0.1))
+    d_v = torch.empty(rows, cols, device="cuda")
+    sums = []
+    for m in (d_g, d_u):
+        L.check(L.lib().dooms_cuda_dequantize(dtype, m.data_ptr(), rows, cols, d_v.data_ptr(), None))
+        sums.append((d_v.double() @ d_x.double(), 2e-6 * (d_v.double().abs() @ d_x.double().abs())))
+    (g, bg), (u, bu) = sums
+    d_h = torch.empty(rows, dtype=torch.float32, device="cuda")
+    taken_by(kernel, lambda: L.check(L.lib().dooms_cuda_gate_up(dtype, d_g.data_ptr(), d_u.data_ptr(), d_x.data_ptr(), d_h.data_ptr(), rows, cols, None)))
+    L.check(L.lib().dooms_cuda_kernel_status(None, None))
+    want = torch.nn.functional.silu(g) * u
+    # silu is 1.1-Lipschitz and at most |g|; exp, divide and the products round to a few ulp
+    assert bool(((d_h.double() - want).abs() <= 1.1 * bg * (u.abs() + bu) + g.abs() * bu + 1e-6 * want.abs() + 1e-30).all())
+
+
 @pytest.mark.parametrize("dtype", MATRIX_TYPES)
 def test_gate_up_matches_the_oracle(dtype):
     rows, cols = 4864, 1024
@@ -101,7 +155,8 @@ def test_gate_up_matches_the_oracle(dtype):
     assert np.sqrt(((got - want) ** 2).sum() / (want ** 2).sum()) < 1e-5
 
 
-@pytest.mark.parametrize("dtype,shape", [(L.Q4_0, (300, 4096)), (L.Q4_0, (1152, 896)), (L.Q4_K, (64, 14336)), (L.Q4_0, (4864, 1024))])
+@pytest.mark.parametrize("dtype,shape", [(L.Q4_0, (300, 4096)), (L.Q4_0, (1152, 896)), (L.Q4_K, (64, 14336)), (L.Q4_0, (4864, 1024)), (L.Q4_0, (6145, 4096)),
+                                         (L.Q4_0, (18977, 896))])
 def test_projections_on_an_input_that_is_already_split_give_the_same_bits(dtype, shape):
     """The integer tensor-core kernel on the split a producer kernel would leave (dooms_cuda_split_input) against the same kernel splitting the f32 input
     itself: identical results, plain and gate / up."""
