@@ -11,27 +11,17 @@
 
 #include <algorithm>
 
+#include "attention_decode_body.cuh"
 #include "kernels.h"
 #include "launch.cuh"
 #include "ptx.cuh"
 #include "xsplit.cuh"
 
+
 namespace dooms {
 namespace cuda {
 
 using namespace dooms::dev;
-
-namespace {
-
-}  // namespace
-}  // namespace cuda
-}  // namespace dooms
-
-#include "attention_decode_body.cuh"
-
-namespace dooms {
-namespace cuda {
-
 using namespace dooms::cuda::attn_decode;
 
 namespace {
@@ -46,7 +36,8 @@ __global__ void __launch_bounds__(kThreads) k_attention_decode(const AttnDecodeP
 
 // Heads of 128 on a context of which a range holds two pairs of tiles at most: two stages, and 74 KB instead of 143, leave a block room beside the projection in
 // front, so that its fetches are early (the 8B shape at 60 keys: 10.3 us to 6.0). Longer ranges want the second pair on its way (the 32B shape
-// at 8200 keys, ranges of four pairs: 24.1 us with four stages, 28.4 with two, also with twice as many blocks).
+// at 8200 keys, ranges of four pairs: 24.1 us with four stages, 28.4 with two, also with twice as many blocks). What counts is the context the decoder was created
+// with: a captured step serves all of its positions.
 template <int D, int GP, int STAGES>
 cudaError_t launch_staged(const AttnDecodeParams & p, cudaStream_t stream) {
     constexpr size_t smem = attention_decode_smem_bytes<D, GP, STAGES>();

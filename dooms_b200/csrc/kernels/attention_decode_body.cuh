@@ -44,25 +44,14 @@ struct AttnDecodeParams {
     int64_t slot_elems;       // f16 elements between the caches of consecutive slots
     int64_t part_row_floats;  // floats of `part` per row
     __half * out16;           // optional: the merged rows as f16 as well ([row][n_head * head_dim]), the tensor-core GEMM's operand
+    int cluster;              // the blocks of kCluster consecutive ranges of a key/value head form a thread-block cluster
     // Single-row decode inside a step whose position was final before this kernel could start (launch_attention_gqa): the cached keys and values of earlier
     // positions do not depend on the projection in front of this kernel, so a block asks for its range before it waits for that projection. The row of the
     // new position is whatever the cache held; it is overwritten in shared memory once the projection is done, as it always was.
-    int cluster;              // the blocks of kCluster consecutive ranges of a key/value head form a thread-block cluster
     int cache_ready;          // the positions the caches have room for (0: not so)
 };
 
 __device__ __forceinline__ void cp16(uint32_t dst, const void * src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void cluster_barrier() {      // all threads of the cluster's blocks that have not left
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {      // the float at shared-memory address addr of block `rank` of the cluster
-    uint32_t at;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
-    return v;
-}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t & r0, uint32_t & r1, uint32_t & r2, uint32_t & r3) {

@@ -37,17 +37,6 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
 }
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) { const __half2 h = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t *>(&h); }
 
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {      // the float at shared-memory address addr of block `rank` of the cluster
-    uint32_t at;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
-    return v;
-}
 // 2^x; results below 2^-126 come out as zero (they are probabilities of a softmax whose largest is 1, rounded to f16 next).
 __device__ __forceinline__ float ex2(float x) {
     float y;

@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
     const int tile = p.tile0 + int(blockIdx.x);
     const int64_t n0 = int64_t(tile % p.tiles_n) * (pair ? 2 * kRowsW : kRowsW);
     const int m0 = (tile / p.tiles_n) * p.T;
-    // a share of the reduction (f16-row path only): k steps ks0 .. ks0 + ksteps - 1
+    // a share of the reduction (f16 rows: of whole k steps; wide producers: of whole 256-element groups): k steps ks0 .. ks0 + ksteps - 1
     const int ks0 = p.ks_per > 0 ? int(blockIdx.z) * p.ks_per : 0;
     const int ksteps = p.ks_per > 0 ? min(p.K / kStepK - ks0, p.ks_per) : p.K / kStepK;
     const uint32_t ncols = uint32_t(p.T) * NMAT;      // the second accumulator starts T columns behind the first

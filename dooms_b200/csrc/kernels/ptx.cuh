@@ -1,5 +1,5 @@
 #pragma once
-// Thin wrappers over the sm_100a PTX this backend uses directly: mbarriers, 1-D bulk (TMA) copies into shared memory, warp-level integer MMA.
+// Thin wrappers over the sm_100a PTX this backend uses directly: mbarriers, 1-D bulk (TMA) copies into shared memory, clusters, warp-level integer MMA.
 // Every copy here targets the issuing block only. Every wait is bounded: it gives up after a fixed number of polls and reports failure to the caller.
 #include <cstdint>
 
@@ -33,6 +33,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 // Global -> shared bulk copy: both addresses 16-byte aligned, bytes a multiple of 16; completion is counted on the mbarrier.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// Thread-block clusters: a barrier of all threads of the cluster's blocks that have not left, and the float at shared-memory address addr of block `rank`.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {
+    uint32_t at;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
 }
 
 // D(16x8, s32) += A(16x32, s8, row) * B(32x8, s8, col). Fragments (g = lane / 4, t = lane % 4): a0 / a2 = row g, k 4t..4t+3 / 16+4t..; a1 / a3 = row g + 8;
